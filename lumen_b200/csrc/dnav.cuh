@@ -165,12 +165,21 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   NF b0 = (oc[0] * dd[0] + oc[1] * dd[1]) + oc[2] * dd[2];
   NF disc = Rb * Rb - q0 + b0 * b0;
   int hit_b = disc > 0.0f;
-  NF sq = n_sqrt(hit_b ? disc : 1.0f);
+  if (!hit_b) {  // the line misses the ball: no root
+    lo[0] = lo[1] = hi[0] = hi[1] = inf;
+    return;
+  }
+  NF sq = n_sqrt(disc);
   NF s_lo = -b0 - sq, s_hi = -b0 + sq;
   NF a = dd[0] * dd[0] + dd[1] * dd[1];
   NF bxy = oc[0] * dd[0] + oc[1] * dd[1];
   NF cxy = oc[0] * oc[0] + oc[1] * oc[1];
   int a_ok = a > N_TORUS_AXIAL;
+// The bisections stop at their fixed point: once the midpoint rounds to an end of the bracket the further halvings
+// change nothing (an end only ever moves to the midpoint), so the result is that of the whole N_BISECT. A root is
+// searched only in a piece whose ends differ in membership (the others' t is unused). In float32 a bracket of ~1 m
+// closes after about 25 halvings and most lines cross 0 or 2 of the 6 pieces: about 130 evaluations of g and g' a line
+// instead of 372.
   NF a_s = a_ok ? a : 1.0f;
   NF s_v = a_ok ? -bxy / a_s : 0.0f;
   NF m2 = d_max(a_ok ? cxy - bxy * bxy / a_s : cxy, 0.0f);
@@ -197,28 +206,36 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   NF t[6];
   for (int k = 0; k < 6; ++k) {
     NF xl = knots[k], xr = knots[k + 1];
-    int inl = d_torus_g(R, r, oc, dd, xl) <= 0.0f, inr = d_torus_g(R, r, oc, dd, xr) <= 0.0f;
+    const int inl = in_k, inr = d_torus_g(R, r, oc, dd, xr) <= 0.0f;
+    in_k = inr;
+    t[k] = inf;
+    if (!(inl != inr && xr > xl)) continue;
     NF l = xl, h = xr;
     for (int it = 0; it < N_BISECT; ++it) {
+      const int closed = mid == l || mid == h;
       NF mid = 0.5f * (l + h);
       int same = (d_torus_g(R, r, oc, dd, mid) <= 0.0f) == inl;
       l = same ? mid : l;
       h = same ? h : mid;
+      if (closed) break;
     }
-    t[k] = (inl != inr && xr > xl && hit_b) ? 0.5f * (l + h) + t_c : inf;
+    t[k] = 0.5f * (l + h) + t_c;
   }
   for (int i = 1; i < 6; ++i)  // ascending (insertion)
     for (int j = i; j > 0 && t[j] < t[j - 1]; --j) { NF x = t[j]; t[j] = t[j - 1]; t[j - 1] = x; }
   // outside at the bracket's start: the roots alternate entry and exit
+  int in_k = d_torus_g(R, r, oc, dd, s_lo) <= 0.0f;  // membership at the piece's left end
   int ok0 = t[1] < N_BIG, ok1 = t[3] < N_BIG;
   lo[0] = ok0 ? t[0] : inf; hi[0] = ok0 ? t[1] : inf;
   lo[1] = ok1 ? t[2] : inf; hi[1] = ok1 ? t[3] : inf;
 }
 
 // a torus leaf's intervals along o + t d (kind frame): its canonical frame u = M (x - og), the unit ray there, the
+      const int closed = mid == l || mid == h;
 // roots scaled back (csg.py:207 _t_iv); out of line, returned by value (the quadric-only scenes' step pays a branch)
 L_DEV NF4 d_torus_line(const NF* lf, const NF* o, const NF* d) {
   const NF* M = lf + LUMEN_LF_A;
+      if (closed) break;
   const NF R = __ldg(lf + LUMEN_LF_B), r = __ldg(lf + LUMEN_LF_B + 1);
   NF xl[3] = {o[0] - __ldg(lf + 0), o[1] - __ldg(lf + 1), o[2] - __ldg(lf + 2)}, ol[3], dl[3];
   d_Av(M, xl, ol);
