@@ -79,6 +79,130 @@ static int upload_raw(LumenScene* sc, const void* h, size_t bytes, void** out) {
     field = (decltype(field))p_;                                                    \
   } while (0)
 
+// The ray traversal's own tree over the leaves of each volume's BVH, in the node records of DScene::node_w (root at
+// the volume's first node, the other inner nodes after the scene's): built by the surface area heuristic, which takes
+// the expected box tests of a random ray instead of the equal halves a caller's tree may have. The queries find the
+// same event over any tree (every leaf box a ray meets before the best event is visited); the boxes are the leaves'
+// own. No deeper than the traversal's stack: a split that could not finish within it is the median's.
+struct RayTree {
+  struct Box { float v[6]; };
+  std::vector<Box> box;
+  std::vector<int> code, weight, id;
+  std::vector<float>* rec;
+
+  static Box none() {
+    const float i = std::numeric_limits<float>::infinity();
+    return {{i, i, i, -i, -i, -i}};
+  }
+  static void grow(Box& a, const Box& b) {
+    for (int k = 0; k < 3; ++k) {
+      a.v[k] = std::min(a.v[k], b.v[k]);
+      a.v[3 + k] = std::max(a.v[3 + k], b.v[3 + k]);
+    }
+  }
+  static double area(const Box& b) {
+    const double x = (double)b.v[3] - b.v[0], y = (double)b.v[4] - b.v[1], z = (double)b.v[5] - b.v[2];
+    return x < 0 || y < 0 || z < 0 ? 0.0 : x * y + y * z + z * x;
+  }
+  static int levels(int m) {  // of a balanced tree over m leaves
+    int l = 1;
+    while (((long long)1 << (l - 1)) < m) ++l;
+    return l;
+  }
+  double centre(int i, int ax) const { return 0.5 * ((double)box[i].v[ax] + box[i].v[3 + ax]); }
+  void order(int a, int b, int ax) {
+    std::sort(id.begin() + a, id.begin() + b, [&](int p, int q) {
+      const double cp = centre(p, ax), cq = centre(q, ax);
+      return cp != cq ? cp < cq : p < q;
+    });
+  }
+
+  // writes the record of the inner node over id[a, b) (at least two leaves) at record `at` and returns its box
+  Box build(int a, int b, int at, int level) {
+    const int n = b - a;
+    int split = a + n / 2, best_ax = -1;
+    double best = std::numeric_limits<double>::infinity();
+    std::vector<double> right(n);
+    for (int ax = 0; ax < 3; ++ax) {
+      order(a, b, ax);
+      Box r = none();
+      double wr = 0.0;
+      for (int i = n - 1; i > 0; --i) {
+        grow(r, box[id[a + i]]);
+        wr += weight[id[a + i]];
+        right[i] = area(r) * wr;
+      }
+      Box l = none();
+      double wl = 0.0;
+      for (int i = 1; i < n; ++i) {
+        grow(l, box[id[a + i - 1]]);
+        wl += weight[id[a + i - 1]];
+        const double cost = area(l) * wl + right[i];
+        if (cost < best && level + levels(std::max(i, n - i)) <= LUMEN_MAX_BVH_DEPTH) {
+          best = cost;
+          split = a + i;
+          best_ax = ax;
+        }
+      }
+    }
+    if (best_ax < 0) best_ax = 2;  // the last axis' order is there: the median
+    if (best_ax != 2) order(a, b, best_ax);
+    Box all = none();
+    float r[16];
+    memset(r, 0, sizeof(r));
+    for (int side = 0; side < 2; ++side) {
+      const int p = side ? split : a, q = side ? b : split;
+      Box bx;
+      int c;
+      if (q - p == 1) {
+        bx = box[id[p]];
+        c = code[id[p]];
+      } else {
+        c = (int)(rec->size() / 16);
+        rec->resize(rec->size() + 16);
+        bx = build(p, q, c, level + 1);
+      }
+      memcpy(r + 6 * side, bx.v, sizeof(bx.v));
+      memcpy(r + 12 + side, &c, 4);
+      grow(all, bx);
+    }
+    memcpy(r + 14, &at, 4);
+    memcpy(rec->data() + (size_t)at * 16, r, sizeof(r));
+    return all;
+  }
+};
+
+static void ray_records(const LumenSceneDesc* d, std::vector<float>& rec, std::vector<int32_t>& witem) {
+  rec.assign((size_t)d->n_node * 16, 0.0f);
+  for (int v = 0; v <= d->n_vol; ++v) {
+    const int n0 = d->vol_i[(size_t)v * LUMEN_VOL_I + LUMEN_VI_NODE0], n1 = d->vol_i[(size_t)v * LUMEN_VOL_I + LUMEN_VI_NODE1];
+    if (n0 >= n1) continue;
+    RayTree t;
+    t.rec = &rec;
+    std::vector<int> todo{n0};
+    while (!todo.empty()) {  // the leaves: their boxes, and their items as a list ended by -1
+      const int nd = todo.back();
+      todo.pop_back();
+      const int32_t* ni = d->node_i + (size_t)nd * LUMEN_NODE_I;
+      if (ni[1] == 0) {
+        todo.push_back(nd + 1);
+        todo.push_back(d->node_i[(size_t)(nd + 1) * LUMEN_NODE_I]);
+        continue;
+      }
+      RayTree::Box b;
+      memcpy(b.v, d->node_f + (size_t)nd * LUMEN_NODE_F, sizeof(b.v));
+      t.id.push_back((int)t.box.size());
+      t.box.push_back(b);
+      t.weight.push_back(ni[1]);
+      t.code.push_back(-2 - (int)witem.size());
+      for (int k = 0; k < ni[1]; ++k) witem.push_back(d->items[ni[2] + k]);
+      witem.push_back(-1);
+    }
+    if (t.id.size() == 1) memcpy(rec.data() + (size_t)n0 * 16 + 14, &t.code[0], 4);
+    else t.build(0, (int)t.id.size(), n0, 1);
+  }
+}
+
 static void value_roles(const LumenSceneDesc* d, std::vector<std::pair<int, int>>& out);
 static int check_values(const std::vector<std::pair<int, int>>& roles, const int32_t* tab, int n_tab, const float* pool);
 
@@ -780,44 +904,14 @@ int32_t lumen_b200_scene_create(const LumenSceneDesc* d, LumenScene** out) {
   UPLOAD(S.node_i, d->node_i, (size_t)d->n_node * LUMEN_NODE_I);
   UPLOAD(S.items, d->items, (size_t)d->n_item);
   {  // the float32 ray traversal's node records (DScene::node_w) and the leaves' item lists
-    const int nn = d->n_node;
-    std::vector<int32_t> code((size_t)(nn > 0 ? nn : 1), -1), witem;
-    for (int n = 0; n < nn; ++n) {
-      const int32_t* ni = d->node_i + (size_t)n * LUMEN_NODE_I;
-      if (ni[1] > 0 && (ni[2] < 0 || ni[2] + ni[1] > d->n_item)) {
-        code[n] = -1;  // outside every BVH the checks above walked: never reached
-      } else if (ni[1] > 0) {
-        code[n] = -2 - (int32_t)witem.size();
-        for (int k = 0; k < ni[1]; ++k) witem.push_back(d->items[ni[2] + k]);
-        witem.push_back(-1);
-      } else {
-        code[n] = n;
-      }
-    }
-    // a record without children (a leaf's, or a node outside every BVH) has NaN boxes, which no slab test meets
-    // (every comparison with NaN is false), and codes -1
-    std::vector<float> rec((size_t)(nn > 0 ? nn : 1) * 16, std::numeric_limits<float>::quiet_NaN());
-    for (int n = 0; n < nn; ++n) {
-      float* r = rec.data() + (size_t)n * 16;
-      const int32_t none = -1, zero = 0;
-      memcpy(r + 12, &none, 4);
-      memcpy(r + 13, &none, 4);
-      memcpy(r + 15, &zero, 4);
-      const int lc = n + 1, rc = lc < nn ? d->node_i[(size_t)lc * LUMEN_NODE_I] : -1;
-      if (d->node_i[(size_t)n * LUMEN_NODE_I + 1] == 0 && lc < nn && rc >= 0 && rc < nn) {
-        std::copy(d->node_f + (size_t)lc * LUMEN_NODE_F, d->node_f + (size_t)lc * LUMEN_NODE_F + 6, r);
-        std::copy(d->node_f + (size_t)rc * LUMEN_NODE_F, d->node_f + (size_t)rc * LUMEN_NODE_F + 6, r + 6);
-        memcpy(r + 12, &code[lc], 4);
-        memcpy(r + 13, &code[rc], 4);
-      }
-      memcpy(r + 14, &code[n], 4);
-    }
-    if (nn > 0) {
-      UPLOAD(S.node_w, reinterpret_cast<const float4*>(rec.data()), (size_t)nn * 4);
+    std::vector<float> rec;
+    std::vector<int32_t> witem;
+    ray_records(d, rec, witem);
+    S.node_w = nullptr;
+    S.witem = nullptr;
+    if (!rec.empty()) {
+      UPLOAD(S.node_w, reinterpret_cast<const float4*>(rec.data()), rec.size() / 4);
       UPLOAD(S.witem, witem.data(), witem.size());
-    } else {
-      S.node_w = nullptr;
-      S.witem = nullptr;
     }
   }
   UPLOAD(S.kind_i, d->kind_i, (size_t)d->n_kind * LUMEN_KIND_I);
