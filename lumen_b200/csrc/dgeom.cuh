@@ -58,7 +58,7 @@ struct DScene {
   const float* __restrict__ leaf_f;
   const int32_t* __restrict__ leaf_i;
   const float* __restrict__ plane_f;
-  const int32_t* __restrict__ prog_i;
+  const uint32_t* __restrict__ kind_tt;  // per kind its boolean's truth table over the leaves' memberships, 8 words
   const int32_t* __restrict__ cls_medium;
   const int32_t* __restrict__ cls_born;  // per class the entry class of a sensor counting photons born in it, or null
   const int32_t* __restrict__ pair_pre;  // per class pair 1: the deposit goes to the volume left's sensor, or null

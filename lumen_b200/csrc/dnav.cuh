@@ -51,7 +51,22 @@ L_DEV void d_to_world_dir(const DScene& S, int i, const NF* g, NF* gw) {
 }
 
 // ------------------------------------------------------------------------------------------- leaf intervals
-struct Iv { NF lo0, hi0; int f_lo0, f_hi0; NF lo1, hi1; int f_lo1, f_hi1; };
+// a leaf's interval set along a ray: two slots, and the faces of their ends (0 the quadric or torus, 1 + plane, -1
+// none), a signed byte each in f (byte j: lo0, hi0, lo1, hi1). Packed: the scan of an 8-leaf solid holds its sets in
+// local memory and reads a face only at the one end that wins (5 words a leaf instead of 8).
+struct Iv { NF lo0, hi0, lo1, hi1; int f; };
+L_DEV int iv_pack(int a, int b, int c, int d) {
+  return (a & 0xff) | ((b & 0xff) << 8) | ((c & 0xff) << 16) | (int)((unsigned)d << 24);
+}
+L_DEV int iv_face(int f, int j) { return (int)(int8_t)((unsigned)f >> (8 * j)); }
+// the slots swapped where the first is empty and the second is not
+L_DEV Iv iv_ordered(NF lo0, NF hi0, int f0, int g0, NF lo1, NF hi1, int f1, int g1, int swap) {
+  Iv r;
+  r.lo0 = swap ? lo1 : lo0; r.hi0 = swap ? hi1 : hi0;
+  r.lo1 = swap ? lo0 : lo1; r.hi1 = swap ? hi0 : hi1;
+  r.f = swap ? iv_pack(f1, g1, f0, g0) : iv_pack(f0, g0, f1, g1);
+  return r;
+}
 
 L_DEV void d_Av(const NF* A, const NF* v, NF* out) {
 #pragma unroll
@@ -156,6 +171,11 @@ L_DEV int d_torus_meets(NF R, NF r, const NF* ol, const NF* du) {
   return meet && r2_min <= r_out * r_out && r2_max >= r_in * r_in;
 }
 
+// The bisections stop at their fixed point: once the midpoint rounds to an end of the bracket the further halvings
+// change nothing (an end only ever moves to the midpoint), so the result is that of the whole N_BISECT. A root is
+// searched only in a piece whose ends differ in membership (the others' t is unused). In float32 a bracket of ~1 m
+// closes after about 25 halvings and most lines cross 0 or 2 of the 6 pieces: about 130 evaluations of g and g' a line
+// instead of 372. The solids box, 100,003 photons, persistent loop: 46.5 -> 23.4 ms (with the truth tables below).
 L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) {
   const NF inf = N_HUGE;
   NF t_c = -((od[0] * dd[0] + od[1] * dd[1]) + od[2] * dd[2]);
@@ -175,11 +195,6 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   NF bxy = oc[0] * dd[0] + oc[1] * dd[1];
   NF cxy = oc[0] * oc[0] + oc[1] * oc[1];
   int a_ok = a > N_TORUS_AXIAL;
-// The bisections stop at their fixed point: once the midpoint rounds to an end of the bracket the further halvings
-// change nothing (an end only ever moves to the midpoint), so the result is that of the whole N_BISECT. A root is
-// searched only in a piece whose ends differ in membership (the others' t is unused). In float32 a bracket of ~1 m
-// closes after about 25 halvings and most lines cross 0 or 2 of the 6 pieces: about 130 evaluations of g and g' a line
-// instead of 372.
   NF a_s = a_ok ? a : 1.0f;
   NF s_v = a_ok ? -bxy / a_s : 0.0f;
   NF m2 = d_max(a_ok ? cxy - bxy * bxy / a_s : cxy, 0.0f);
@@ -194,16 +209,19 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
     NF l = el[k], h = eh[k];
     for (int it = 0; it < N_BISECT; ++it) {
       NF mid = 0.5f * (l + h);
+      const int closed = mid == l || mid == h;
       NF gm = d_torus_dg(R, oc, dd, mid);
       int right = k == 1 ? gm > 0.0f : gm < 0.0f;
       l = right ? mid : l;
       h = right ? h : mid;
+      if (closed) break;
     }
     e[k] = 0.5f * (l + h);
   }
   // the roots: one per monotone piece whose ends differ in membership
   const NF knots[7] = {s_lo, e[0], p1, e[1], p2, e[2], s_hi};
   NF t[6];
+  int in_k = d_torus_g(R, r, oc, dd, s_lo) <= 0.0f;  // membership at the piece's left end
   for (int k = 0; k < 6; ++k) {
     NF xl = knots[k], xr = knots[k + 1];
     const int inl = in_k, inr = d_torus_g(R, r, oc, dd, xr) <= 0.0f;
@@ -212,8 +230,8 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
     if (!(inl != inr && xr > xl)) continue;
     NF l = xl, h = xr;
     for (int it = 0; it < N_BISECT; ++it) {
-      const int closed = mid == l || mid == h;
       NF mid = 0.5f * (l + h);
+      const int closed = mid == l || mid == h;
       int same = (d_torus_g(R, r, oc, dd, mid) <= 0.0f) == inl;
       l = same ? mid : l;
       h = same ? h : mid;
@@ -224,18 +242,15 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   for (int i = 1; i < 6; ++i)  // ascending (insertion)
     for (int j = i; j > 0 && t[j] < t[j - 1]; --j) { NF x = t[j]; t[j] = t[j - 1]; t[j - 1] = x; }
   // outside at the bracket's start: the roots alternate entry and exit
-  int in_k = d_torus_g(R, r, oc, dd, s_lo) <= 0.0f;  // membership at the piece's left end
   int ok0 = t[1] < N_BIG, ok1 = t[3] < N_BIG;
   lo[0] = ok0 ? t[0] : inf; hi[0] = ok0 ? t[1] : inf;
   lo[1] = ok1 ? t[2] : inf; hi[1] = ok1 ? t[3] : inf;
 }
 
 // a torus leaf's intervals along o + t d (kind frame): its canonical frame u = M (x - og), the unit ray there, the
-      const int closed = mid == l || mid == h;
 // roots scaled back (csg.py:207 _t_iv); out of line, returned by value (the quadric-only scenes' step pays a branch)
 L_DEV NF4 d_torus_line(const NF* lf, const NF* o, const NF* d) {
   const NF* M = lf + LUMEN_LF_A;
-      if (closed) break;
   const NF R = __ldg(lf + LUMEN_LF_B), r = __ldg(lf + LUMEN_LF_B + 1);
   NF xl[3] = {o[0] - __ldg(lf + 0), o[1] - __ldg(lf + 1), o[2] - __ldg(lf + 2)}, ol[3], dl[3];
   d_Av(M, xl, ol);
@@ -254,16 +269,8 @@ L_CALL Iv d_torus_iv(const NF* lf, NF3 ov, NF3 dv) {
   const NF o[3] = {ov.x, ov.y, ov.z}, d[3] = {dv.x, dv.y, dv.z};
   NF4 tv = d_torus_line(lf, o, d);
   const NF inf = N_HUGE;
-  Iv r;
-  int ok0 = tv.x < tv.y, ok1 = tv.z < tv.w;
-  r.lo0 = ok0 ? tv.x : inf; r.hi0 = ok0 ? tv.y : inf; r.f_lo0 = ok0 ? 0 : -1; r.f_hi0 = ok0 ? 0 : -1;
-  r.lo1 = ok1 ? tv.z : inf; r.hi1 = ok1 ? tv.w : inf; r.f_lo1 = ok1 ? 0 : -1; r.f_hi1 = ok1 ? 0 : -1;
-  if (!ok0 && ok1) {
-    Iv s = r;
-    r.lo0 = s.lo1; r.hi0 = s.hi1; r.f_lo0 = s.f_lo1; r.f_hi0 = s.f_hi1;
-    r.lo1 = s.lo0; r.hi1 = s.hi0; r.f_lo1 = s.f_lo0; r.f_hi1 = s.f_hi0;
-  }
-  return r;
+  const int ok0 = tv.x < tv.y, ok1 = tv.z < tv.w, f0 = ok0 ? 0 : -1, f1 = ok1 ? 0 : -1;
+  return iv_ordered(ok0 ? tv.x : inf, ok0 ? tv.y : inf, f0, f0, ok1 ? tv.z : inf, ok1 ? tv.w : inf, f1, f1, !ok0 && ok1);
 }
 
 // whether the torus holds x (kind frame): (rho - R)^2 + z^2 <= r^2 in its canonical frame (csg.py:301 _inside_leaf)
@@ -301,27 +308,12 @@ L_DEV Iv d_leaf_iv(const DScene& S, int g, const NF* o, const NF* d) {
   NF L0 = -inf, R0 = inf, L1 = inf, R1 = -inf;
   int L0q = 0, R0q = 0;
   if (has_q) d_quad_line(lf, y, d, &L0, &R0, &L0q, &R0q, &L1, &R1);
-  Iv r;
-  {
-    NF lo = d_max(L0, t0p), hi = d_min(R0, t1p);
-    int flo = L0 > t0p ? (L0q ? 0 : f0p) : f0p;
-    int fhi = R0 < t1p ? (R0q ? 0 : f1p) : f1p;
-    int ok = lo < hi && !ep;
-    r.lo0 = ok ? lo : inf; r.hi0 = ok ? hi : inf; r.f_lo0 = ok ? flo : -1; r.f_hi0 = ok ? fhi : -1;
-  }
-  {
-    NF lo = d_max(L1, t0p), hi = d_min(R1, t1p);
-    int flo = L1 > t0p ? 0 : f0p;
-    int fhi = f1p;
-    int ok = lo < hi && !ep;
-    r.lo1 = ok ? lo : inf; r.hi1 = ok ? hi : inf; r.f_lo1 = ok ? flo : -1; r.f_hi1 = ok ? fhi : -1;
-  }
-  if (r.lo0 >= inf && r.lo1 < inf) {
-    Iv s = r;
-    r.lo0 = s.lo1; r.hi0 = s.hi1; r.f_lo0 = s.f_lo1; r.f_hi0 = s.f_hi1;
-    r.lo1 = s.lo0; r.hi1 = s.hi0; r.f_lo1 = s.f_lo0; r.f_hi1 = s.f_hi0;
-  }
-  return r;
+  const NF lo0 = d_max(L0, t0p), hi0 = d_min(R0, t1p), lo1 = d_max(L1, t0p), hi1 = d_min(R1, t1p);
+  const int ok0 = lo0 < hi0 && !ep, ok1 = lo1 < hi1 && !ep;
+  const NF a0 = ok0 ? lo0 : inf, a1 = ok1 ? lo1 : inf;
+  return iv_ordered(a0, ok0 ? hi0 : inf, ok0 ? (L0 > t0p ? (L0q ? 0 : f0p) : f0p) : -1,
+                    ok0 ? (R0 < t1p ? (R0q ? 0 : f1p) : f1p) : -1, a1, ok1 ? hi1 : inf,
+                    ok1 ? (L1 > t0p ? 0 : f0p) : -1, ok1 ? f1p : -1, a0 >= inf && a1 < inf);
 }
 
 L_DEV int d_inside_leaf(const DScene& S, int g, const NF* x) {
@@ -344,25 +336,20 @@ L_DEV int d_inside_leaf(const DScene& S, int g, const NF* x) {
   return pl && qv <= 0.0f;
 }
 
-// the kind's postfix program over a membership functor
-template <class F>
-L_DEV int d_program(const DScene& S, int kind, F member) {
-  const int32_t* k = S.kind_i + (size_t)kind * LUMEN_KIND_I;
-  int p0 = __ldg(k + 2), pl = __ldg(k + 3);
-  int32_t s = 0;
-  for (int p = 0; p < pl; ++p) {
-    int op = __ldg(S.prog_i + (size_t)(p0 + p) * 2), arg = __ldg(S.prog_i + (size_t)(p0 + p) * 2 + 1);
-    int32_t bb = s & 1, aa = (s >> 1) & 1;
-    int32_t r = op == 1 ? (aa | bb) : (op == 2 ? (aa & bb) : (aa & (1 - bb)));
-    if (op == 0) s = (s << 1) | (member(arg) & 1);
-    else s = ((s >> 2) << 1) | r;
-  }
-  return (s & 1) == 1;
+// The kind's postfix program as its truth table over the leaves' memberships (bit l of m: leaf l), built by
+// scene_create: one load instead of an interpreted loop of two dependent loads an operation (the field cage of the
+// liquid-argon box: 7 operations, evaluated at about five points a ray; with the packed sets above, the box's 131,072
+// photons with two tangents 51.3 -> 46.4 ms).
+L_DEV int d_bool(const DScene& S, int kind, unsigned m) {
+  return (__ldg(S.kind_tt + (size_t)kind * (1u << LUMEN_MAX_LEAVES) / 32 + (m >> 5)) >> (m & 31u)) & 1u;
 }
 
 L_DEV int d_inside_kind(const DScene& S, int kind, const NF* x) {
-  int l0 = __ldg(S.kind_i + (size_t)kind * LUMEN_KIND_I);
-  return d_program(S, kind, [&](int l) { return d_inside_leaf(S, l0 + l, x); });
+  const int32_t* k = S.kind_i + (size_t)kind * LUMEN_KIND_I;
+  const int l0 = __ldg(k), nl = __ldg(k + 1);
+  unsigned m = 0;
+  for (int l = 0; l < nl; ++l) m |= (unsigned)d_inside_leaf(S, l0 + l, x) << l;
+  return d_bool(S, kind, m);
 }
 
 // ----------------------------------------------------------------------------------------- first_change
@@ -394,12 +381,14 @@ L_DEV int d_mem_at(const DScene& S, const ScanT<NLMAX>& s, NF t, int use_on) {
     if (on && s.on_leaf == 0 && t < s.hend) m = s.on_inside;
     return m;
   }
-  return d_program(S, s.kind, [&](int l) {
+  unsigned mask = 0;
+  for (int l = 0; l < s.nl; ++l) {
     const Iv& v = s.iv[l];
     int m = (v.lo0 <= t && t < v.hi0) || (v.lo1 <= t && t < v.hi1);
     if (on && l == s.on_leaf && t < s.hend) m = s.on_inside;
-    return m;
-  });
+    mask |= (unsigned)(m & 1) << l;
+  }
+  return d_bool(S, s.kind, mask);
 }
 
 // TORUS: the geometry instantiation: 1 reads torus leaves, mesh chunks and protrusion clips (scenes without them run
@@ -428,23 +417,28 @@ L_DEV void d_scan_init(const DScene& S, ScanT<NLMAX>& s, int kind, const NF* o, 
 struct First { int hit; NF t; int inside, leaf, face; };
 struct Fc { int hit; NF t; int inside, leaf, face, inside0; First first; };
 
+// the nearest end past t_cur (t_cur >= 0): its t, leaf, face and whether it is an entry; the face on the skipped leaf
+// alone is read along the way
 template <int NLMAX>
 L_DEV void d_nearest(const ScanT<NLMAX>& s, NF t_cur, NF* e1o, int* lbo, int* fco, int* eko) {
-  NF e1 = N_HUGE;
-  int lb = -1, fc = -1, ek = 0;
+  NF e1 = N_BIG;
+  int lb = -1, jb = 0;
   for (int l = 0; l < (NLMAX == 1 ? 1 : s.nl); ++l) {
     const Iv& v = s.iv[l];
+    const int skip = s.has_skip && l == s.skip_leaf;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      NF ep = j == 0 ? v.lo0 : (j == 1 ? v.hi0 : (j == 2 ? v.lo1 : v.hi1));
-      int fp = j == 0 ? v.f_lo0 : (j == 1 ? v.f_hi0 : (j == 2 ? v.f_lo1 : v.f_hi1));
-      int en = (j & 1) == 0;
-      int ok = n_abs(ep) < N_BIG && ep <= s.t1 && ep > t_cur && ep < e1;
-      if (s.has_skip) ok = ok && !(l == s.skip_leaf && fp == s.skip_face && s.skip_entry == en && ep < s.skip_thi);
-      if (ok) { e1 = ep; lb = l; fc = fp; ek = en; }
+      const NF ep = j == 0 ? v.lo0 : (j == 1 ? v.hi0 : (j == 2 ? v.lo1 : v.hi1));
+      int ok = ep <= s.t1 && ep > t_cur && ep < e1;
+      if (skip)
+        ok = ok && !(iv_face(v.f, j) == s.skip_face && s.skip_entry == ((j & 1) == 0) && ep < s.skip_thi);
+      if (ok) { e1 = ep; lb = l; jb = j; }
     }
   }
-  *e1o = e1; *lbo = lb; *fco = fc; *eko = ek;
+  *e1o = lb >= 0 ? e1 : N_HUGE;
+  *lbo = lb;
+  *fco = lb >= 0 ? iv_face(s.iv[NLMAX == 1 ? 0 : lb].f, jb) : -1;
+  *eko = lb >= 0 && (jb & 1) == 0;
 }
 
 template <int NLMAX>
@@ -1078,13 +1072,13 @@ L_DEV Best d_enter_x(const DScene& S, const Ctx& c, int has_own, int vi) {
 // eleven). The two differ for a NaN, which no finite ray and box give, and in a zero's sign, which no comparison sees.
 // With scene_create's tree (ray_records) the tank's 2^24 photons take 45.6 instead of 51.6 ms.
 L_DEV void d_slab_box(const float* bx, const NF* o, const NF* inv, NF* tin, NF* tout) {
-#endif
   const NF ax = (bx[0] - o[0]) * inv[0], bxx = (bx[3] - o[0]) * inv[0];
   const NF ay = (bx[1] - o[1]) * inv[1], by = (bx[4] - o[1]) * inv[1];
   const NF az = (bx[2] - o[2]) * inv[2], bz = (bx[5] - o[2]) * inv[2];
   *tin = fmaxf(fmaxf(fminf(ax, bxx), fminf(ay, by)), fminf(az, bz));
   *tout = fminf(fminf(fmaxf(ax, bxx), fmaxf(ay, by)), fmaxf(az, bz));
 }
+#endif
 
 // The candidate entries of volume c.v along the ray (navigate.py:482 enter, :465 _group, :430 _node): the volume's own
 // solid first (has_own), then its BVH depth first, the nearer child first and the farther onto the stack with its

@@ -79,6 +79,27 @@ static int upload_raw(LumenScene* sc, const void* h, size_t bytes, void** out) {
     field = (decltype(field))p_;                                                    \
   } while (0)
 
+// Each kind's postfix boolean as a truth table over its leaves' memberships: bit m of the kind's 2^LUMEN_MAX_LEAVES
+// bits is the program's value where leaf l holds the point for every bit l of m.
+static std::vector<uint32_t> truth_tables(const LumenSceneDesc* d) {
+  const int bits = 1 << LUMEN_MAX_LEAVES, words = bits / 32;
+  std::vector<uint32_t> tt((size_t)(d->n_kind > 0 ? d->n_kind : 1) * words, 0u);
+  for (int k = 0; k < d->n_kind; ++k) {
+    const int32_t* ki = d->kind_i + (size_t)k * LUMEN_KIND_I;
+    for (int m = 0; m < (1 << ki[1]); ++m) {
+      uint32_t s = 0;
+      for (int p = 0; p < ki[3] && ki[2] >= 0 && ki[2] + p < d->n_prog; ++p) {
+        const int32_t* pr = d->prog_i + (size_t)(ki[2] + p) * LUMEN_PROG_I;
+        const uint32_t b = s & 1u, a = (s >> 1) & 1u;
+        if (pr[0] == 0) s = (s << 1) | (((uint32_t)m >> (pr[1] & 31)) & 1u);
+        else s = ((s >> 2) << 1) | (pr[0] == 1 ? (a | b) : (pr[0] == 2 ? (a & b) : (a & (1u - b))));
+      }
+      if (s & 1u) tt[(size_t)k * words + m / 32] |= 1u << (m % 32);
+    }
+  }
+  return tt;
+}
+
 // The ray traversal's own tree over the leaves of each volume's BVH, in the node records of DScene::node_w (root at
 // the volume's first node, the other inner nodes after the scene's): built by the surface area heuristic, which takes
 // the expected box tests of a random ray instead of the equal halves a caller's tree may have. The queries find the
@@ -927,7 +948,10 @@ int32_t lumen_b200_scene_create(const LumenSceneDesc* d, LumenScene** out) {
   }
   UPLOAD(S.leaf_i, d->leaf_i, (size_t)d->n_leaf * LUMEN_LEAF_I);
   UPLOAD(S.plane_f, d->plane_f, (size_t)d->n_plane * LUMEN_PLANE_F);
-  UPLOAD(S.prog_i, d->prog_i, (size_t)d->n_prog * LUMEN_PROG_I);
+  {
+    const std::vector<uint32_t> tt = truth_tables(d);
+    UPLOAD(S.kind_tt, tt.data(), tt.size());
+  }
   sc->nav64 = d->precision == LUMEN_PREC_FLOAT64;
   sc->vol_f32 = S.vol_f;
   if (sc->nav64) {  // the float64 navigator reads its arrays through the same pointers (checked non-null above)
