@@ -18,11 +18,12 @@ namespace lb {
 
 enum { STRAIGHT = 0, REFRACT, SPECULAR, BACKSCATTER, GLOSSY, DIFFUSE, N_OUT };
 
-L_DEV float d_tab(const DScene& S, const float* __restrict__ pool, int t, float E) {
-  int off = __ldg(S.tab + 2 * t), k = __ldg(S.tab + 2 * t + 1);
-  const float* xe = pool + off;
-  const float* fv = pool + off + k;
-  if (k == 1 || E <= __ldg(xe)) return __ldg(fv);
+// a table of two knots or more: out of line (about thirty call sites in the step; the step kernel waits on instruction
+// fetch, and a constant's table, the common one, needs two loads). Ground-wall tank with four tangents and a held
+// reference, 2,000,000 photons: 20.9 -> 19.7 ms
+L_CALL float d_tab_k(const float* __restrict__ xe, int k, float E) {
+  const float* fv = xe + k;
+  if (E <= __ldg(xe)) return __ldg(fv);
   if (E >= __ldg(xe + k - 1)) return __ldg(fv + k - 1);
   int i = 1;
   while (i < k - 1 && __ldg(xe + i) <= E) ++i;
@@ -31,6 +32,12 @@ L_DEV float d_tab(const DScene& S, const float* __restrict__ pool, int t, float 
   float dx = x1 - x0;
   float df = f1 - f0;
   return f0 + (E - x0) / dx * df;
+}
+L_DEV float d_tab(const DScene& S, const float* __restrict__ pool, int t, float E) {
+  const int2 ok = __ldg(reinterpret_cast<const int2*>(S.tab) + t);
+  const float* xe = pool + ok.x;
+  if (ok.y == 1) return __ldg(xe + 1);
+  return d_tab_k(xe, ok.y, E);
 }
 
 L_DEV float d_rate(float L) { return L >= D_FLT_TINY ? 1.0f / L : 1.0f / D_FLT_TINY; }
