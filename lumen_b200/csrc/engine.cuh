@@ -51,6 +51,34 @@ struct LumenScene {
   // the wavefront's rounds per photon a slot carries, from the last synchronous wavefront call (an estimate for the
   // asynchronous calls' fixed rounds; concurrent calls may overwrite one another's)
   mutable float wave_rpp = 0.0f;
+  // page-locked words the wavefront's rounds publish their live slots in: one a synchronous call at a time, kept for
+  // the scene's later calls (as many as have run at once) and freed with it
+  mutable std::mutex pub_mu;
+  mutable std::vector<unsigned long long*> pub_free;
+};
+
+// one of the scene's published words for the length of a call
+struct PubLease {
+  const LumenScene* sc;
+  unsigned long long* p = nullptr;
+  explicit PubLease(const LumenScene* s) : sc(s) {}
+  int take() {
+    {
+      std::lock_guard<std::mutex> lock(sc->pub_mu);
+      if (!sc->pub_free.empty()) {
+        p = sc->pub_free.back();
+        sc->pub_free.pop_back();
+        return 0;
+      }
+    }
+    CK(cudaHostAlloc((void**)&p, sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped));
+    return 0;
+  }
+  ~PubLease() {  // every path out of a synchronous call has waited for its stream, or left an error on it
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(sc->pub_mu);
+    sc->pub_free.push_back(p);
+  }
 };
 
 // the position's precision of an instantiation: NAV64 = 1 the float64 navigator's (LUMEN_PREC_FLOAT64)
@@ -107,12 +135,13 @@ struct Launch {
   int budget_chunk;  // steps a thread of the persistent loop counts before it adds them to steps_used (1 .. 256)
   Tally T;
   float* truth;  // the photons' analog records (truth rows, LUMEN_F_TRUTH: the ANALOG instantiation), else null
-  // the wavefront's slots a persistent launch resumes before it takes new photons (its drain: one thread a slot), or
-  // wv_W = 0
+  // the wavefront's live slots a persistent launch resumes before it takes new photons (its drain: thread t the slot
+  // wv_list[t], t < *wv_n; wv_W slots in the pool), or wv_W = 0
   const uint32_t* wv_ph;
   const uint32_t* wv_ex;
   const float* wv_dw;
-  const int32_t* wv_act;
+  const int32_t* wv_list;
+  const unsigned* wv_n;
   int wv_W;
   const int32_t* ev_vol;  // per event its start volume (point-like sources: k_event_locate), or null
 };
@@ -121,7 +150,7 @@ struct Launch {
 struct Pick {
   int torus;
   int single;              // every solid a single quadric / plane leaf
-  int clip;                // a protrusion clip (the wavefront's fill locates without the extended rule)
+  int clip;                // a protrusion clip or frame groups: the extended locate
   int groups;              // frame groups: the extended instantiation with their traversal
   int analog;
   int nav64;               // the scene's navigator is float64
@@ -246,15 +275,22 @@ struct WaveExtra {  // what a slot carries besides the photon: its key, event, r
   PhotonTally pt;
 };
 
-struct Wave {
-  uint32_t* ph;     // W x sizeof(Photon) / 4
+struct Wave {  // the records of the navigator's precision NF
+  uint32_t* ph;     // W x sizeof(PhotonT<NF>) / 4
   uint32_t* ex;     // W x sizeof(WaveExtra) / 4
-  uint32_t* pre;    // W x sizeof(Pre) / 4
-  uint32_t* q;      // W x sizeof(Query) / 4
+  uint32_t* pre;    // W x sizeof(PreT<NF>) / 4
+  uint32_t* q;      // W x sizeof(QueryT<NF>) / 4
   float* dw;        // W x LUMEN_MAX_GRAD (gradient runs)
-  int32_t* act;     // W: the slot holds a live photon
-  unsigned long long* live;  // slots live after the last k_wave_step (zeroed before each)
   int W;
+  // the round's live slots in[0, *n_in) and the next round's out[0, *n_out); mid: the same slots after the query, each
+  // block's photons that scatter before their crossing ahead of its others (slot | place in the block's list << 24)
+  const int32_t* in;
+  const unsigned* n_in;
+  int32_t* out;
+  unsigned* n_out;
+  uint32_t* mid;
+  volatile unsigned long long* pub;  // page-locked host memory: (round << 32 | live slots) of a round that starts, or null
+  unsigned round;
 };
 
 template <class T>
@@ -300,9 +336,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
   __syncthreads();
   unsigned c_ph = 0, c_steps = 0, c_dep = 0, c_trunc = 0, c_multi = 0, c_lost = 0;
   int budget_chunk = 0;
-  if constexpr (!ANALOG && !NAV64) {
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
-    if (i < L.wv_W && L.wv_act[i]) {  // a wavefront slot's photon, where its last round left it
+  if constexpr (!ANALOG) {
+    const unsigned t = blockIdx.x * BLOCK + threadIdx.x;
+    if (L.wv_W > 0 && t < *L.wv_n) {  // a wavefront slot's photon, where its last round left it
+      const int i = L.wv_list[t];
       WaveExtra ex;
       wv_ld(L.wv_ph, L.wv_W, i, ph);
       wv_ld(L.wv_ex, L.wv_W, i, ex);
@@ -428,45 +465,126 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
 }
 
 // ------------------------------------------------------------------------------------------------ the wavefront
-// The photon loop as rounds over a pool of W slots held in HBM (launch variant LUMEN_VARIANT_WAVEFRONT): per round,
-// k_wave_query runs every live slot's step up to and including its navigator query, and k_wave_step the rest of the
-// step, the deposit, the photon's end and the slot's refill from the source. Each kernel is a part of the
+// The photon loop as rounds over a pool of W slots held in HBM (launch variant LUMEN_VARIANT_WAVEFRONT): a fill, then per
+// round k_wave_query runs every live slot's step up to and including its navigator query, and k_wave_step the rest of
+// the step, the deposit, the photon's end and the slot's refill from the source. Each kernel is a part of the
 // megakernel's code with its own registers; the state crosses HBM between them, word-major (word k of slot i at
-// buf[k * W + i]) so that every load and store of a warp is one contiguous 128-byte access.
-template <int G, int TORUS>
-__global__ void __launch_bounds__(256, 3) k_wave_query(Launch L, Wave V) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= V.W || !V.act[i]) return;
-  if (L.abort_flag && *(volatile int*)L.abort_flag) return;
-  Photon ph;
+// buf[k * W + i]) so that the loads and stores of neighbouring slots are contiguous.
+//
+// The kernels run over lists of live slots, not over the pool: once the source is spent a photon's end leaves its lane
+// idle for every later round, and with one photon a slot that is from the second round on (measured before the lists:
+// half of the step kernel's lanes in the liquid-argon box and the fog box, a third in the tank). The step kernel
+// appends the slots that go on to the next round's list, and the query kernel orders each block's slots by the event it
+// found, scatterings ahead of crossings, so that all but one warp of a block of the step kernel run one side of that
+// branch. Both keep a block's slots together and in order: neighbours in a list are neighbours in the pool, and a
+// warp's words stay in few sectors (a split of the whole list, which scatters it round by round, took 129 ms instead of
+// 45 for the tank's 2^24 photons).
+//
+// EXT: the locate of scenes with protrusion clips or frame groups; NAV64: the float64 navigator's records. Every scene
+// runs here: the solids box (clips) 100,003 photons 20.2 ms in the persistent loop, 9.4 in the wavefront; the coated
+// panel (float64) 2^20 photons 7.0 and 4.2 ms.
+template <int EXT, class NF>
+__device__ __forceinline__ void wave_new(const Launch& L, int64_t g, PhotonT<NF>& ph, WaveExtra& ex) {
+  Row r;
+  get_row(L, g, r);
+  d_start<EXT>(L.R.S, r, ph);
+  ex.pkey = fold_in(L.key, (uint32_t)(L.first_id + g));
+  ex.w0 = (double)r.w0;
+  ex.ev = r.event;
+  ex.pad = 0;
+  ex.pt.n = 0;
+  ex.pt.pid = (unsigned)g;
+}
+
+// every slot takes a photon: slot i the call's photon i (W at most the call's photons rounded up to a block)
+template <int EXT, int NAV64>
+__global__ void __launch_bounds__(256) k_wave_fill(Launch L, Wave V) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int have = (int)(L.n < (int64_t)V.W ? L.n : (int64_t)V.W);
+  if (i == 0) {
+    *V.n_out = (unsigned)have;
+    *L.next = (unsigned long long)have;
+  }
+  if (i >= have) return;
+  PhotonT<typename NavOf<NAV64>::F> ph;
   WaveExtra ex;
-  wv_ld(V.ph, V.W, i, ph);
-  wv_ld(V.ex, V.W, i, ex);
-  Pre pr;
-  d_pre<(TORUS & 1)>(L.R, ph, ex.pkey, pr);
-  Query q = d_step_query<TORUS>(L.R, ph, pr);
+  wave_new<EXT>(L, i, ph, ex);
   wv_st(V.ph, V.W, i, ph);
-  wv_st(V.pre, V.W, i, pr);
-  wv_st(V.q, V.W, i, q);
+  wv_st(V.ex, V.W, i, ex);
+  for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = 0.0f;
+  V.out[i] = i;
+}
+
+template <int TORUS, int NAV64>
+__global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wave V) {
+  using NF = typename NavOf<NAV64>::F;
+  __shared__ unsigned sh[8];
+  const unsigned n = *V.n_in;
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j == 0) {
+    *V.n_out = 0u;  // last read as the round before's n_in
+    if (V.pub) {
+      *V.pub = ((unsigned long long)V.round << 32) | n;
+      __threadfence_system();
+    }
+  }
+  if (blockIdx.x * blockDim.x >= n) return;
+  if (L.abort_flag && __syncthreads_or(*(volatile int*)L.abort_flag)) return;  // the step kernel ends every slot
+  const int in = j < n;
+  int i = 0, bulk = 0;
+  if (in) {
+    i = V.in[j];
+    PhotonT<NF> ph;
+    Key pkey;
+    wv_ld(V.ph, V.W, i, ph);
+    wv_ld(V.ex, V.W, i, pkey);  // the record's first words
+    PreT<NF> pr;
+    d_pre<(TORUS & 1)>(L.R, ph, pkey, pr);
+    QueryT<NF> q = d_step_query<TORUS>(L.R, ph, pr);
+    wv_st(V.ph, V.W, i, ph);
+    wv_st(V.pre, V.W, i, pr);
+    wv_st(V.q, V.W, i, q);
+    bulk = pr.mr.mu_c > 0.0f && pr.s < q.t;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
+  const unsigned m = __ballot_sync(0xffffffffu, in && bulk);
+  if (lane == 0) sh[warp] = __popc(m);
+  __syncthreads();
+  unsigned before = __popc(m & ((1u << lane) - 1u)), all = 0;  // the block's scatterings ahead of this thread, and all
+  for (int w = 0; w < warps; ++w) {
+    if (w < warp) before += sh[w];
+    all += sh[w];
+  }
+  if (in) {
+    const unsigned at = bulk ? before : all + threadIdx.x - before;
+    V.mid[blockIdx.x * blockDim.x + at] = (uint32_t)i | (threadIdx.x << 24);
+  }
 }
 
 // BORN: the scene has a sensor that counts the photons born inside it (the branch of their first step, which reads
 // none of the query the query kernel made for it; a scene without one runs the kernel compiled without the branch,
 // the branch costs the tank's plain forward 2 % where it is compiled in)
-template <int G, int BORN>
+template <int G, int BORN, int EXT, int NAV64>
 __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
+  using NF = typename NavOf<NAV64>::F;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   __shared__ double sh_health[LUMEN_N_HEALTH];
-  __shared__ unsigned long long sc[LUMEN_N_COUNT + 1][8];
+  __shared__ unsigned long long sc[LUMEN_N_COUNT][8];
+  __shared__ unsigned on[8], base_out;
+  const unsigned n = *V.n_in;
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x * blockDim.x >= n) return;
   if (threadIdx.x < LUMEN_N_HEALTH) sh_health[threadIdx.x] = 0.0;
+  if (threadIdx.x < 8) on[threadIdx.x] = 0u;
   __syncthreads();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int in = i < V.W;
-  int aborted = L.abort_flag && *(volatile int*)L.abort_flag;
-  int act = in && !aborted && V.act[i];
+  const int in = j < n;
+  const int aborted = L.abort_flag && *(volatile int*)L.abort_flag;
+  int act = in && !aborted;
+  const uint32_t mid = act ? V.mid[j] : 0u;
+  const int i = (int)(mid & 0xffffffu);
   unsigned c_ph = 0, c_steps = 0, c_dep = 0, c_trunc = 0, c_multi = 0, c_lost = 0;
-  Photon ph;
+  PhotonT<NF> ph;
   WaveExtra ex;
   float dw[G > 0 ? G : 1], dq[G > 0 ? G : 1];
   Dep dep;
@@ -482,8 +600,8 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
     if (bp != -2) {
       d_born<G>(L.R, ph, dw, bp, dep, dq, an);
     } else {
-      Pre pr;
-      Query q;
+      PreT<NF> pr;
+      QueryT<NF> q;
       wv_ld(V.pre, V.W, i, pr);
       wv_ld(V.q, V.W, i, q);
       d_post<G>(L.R, ph, dw, pr, q, dep, dq, an);
@@ -511,66 +629,72 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
   warp_add(sh_health + LUMEN_H_START, start_w);
   warp_add(sh_health + LUMEN_H_TRUNCATED, trunc_w);
   // the refill: free slots take consecutive photon ids, one atomic per warp
-  int need = in && !act && !aborted;
+  int need = stepped && !act;
   unsigned m = __ballot_sync(FULL, need);
   if (m) {
     int leader = __ffs(m) - 1;
-    unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(L.next, (unsigned long long)__popc(m));
+    unsigned long long base = (unsigned long long)L.n;
+    if (lane == leader && *(volatile unsigned long long*)L.next < (unsigned long long)L.n)
+      base = atomicAdd(L.next, (unsigned long long)__popc(m));
     base = __shfl_sync(FULL, base, leader);
     if (need) {
       unsigned long long g = base + __popc(m & ((1u << lane) - 1u));
       if (g < (unsigned long long)L.n) {
-        Row r;
-        get_row(L, (int64_t)g, r);
-        d_start(L.R.S, r, ph);
-        ex.pkey = fold_in(L.key, (uint32_t)(L.first_id + (int64_t)g));
-        ex.w0 = (double)r.w0;
-        ex.ev = r.event;
-        ex.pad = 0;
-        ex.pt.n = 0;
-        ex.pt.pid = (unsigned)g;
+        wave_new<EXT>(L, (int64_t)g, ph, ex);
         if (G > 0)
           for (int p = 0; p < L.R.P; ++p) dw[p] = 0.0f;
         act = 1;
       }
     }
   }
-  if (in) {
-    if (act) {
-      wv_st(V.ph, V.W, i, ph);
-      wv_st(V.ex, V.W, i, ex);
-      if (G > 0)
-        for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = dw[p];
-    }
-    V.act[i] = act;
+  if (act) {
+    wv_st(V.ph, V.W, i, ph);
+    wv_st(V.ex, V.W, i, ex);
+    if (G > 0)
+      for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = dw[p];
   }
-  // the block's health, counters and live slots: one atomic per block and value
+  // the next round's list: the block's slots that go on, in the order they came in, one atomic a block
+  const unsigned place = mid >> 24;
+  if (act) atomicOr(&on[place >> 5], 1u << (place & 31u));
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned sum = 0;
+    for (int w = 0; w < 8; ++w) sum += __popc(on[w]);
+    base_out = sum ? atomicAdd(V.n_out, sum) : 0u;
+  }
+  __syncthreads();
+  if (act) {
+    unsigned at = base_out + __popc(on[place >> 5] & ((1u << (place & 31u)) - 1u));
+    for (unsigned w = 0; w < place >> 5; ++w) at += __popc(on[w]);
+    V.out[at] = i;
+  }
+  // the block's health and counters: one atomic per block and value
   const int warp = threadIdx.x >> 5;
-  unsigned long long cv[LUMEN_N_COUNT + 1] = {};
+  unsigned long long cv[LUMEN_N_COUNT] = {};
   cv[LUMEN_C_PHOTONS] = c_ph;
   cv[LUMEN_C_STEPS] = c_steps;
   cv[LUMEN_C_DEPOSITS] = c_dep;
   cv[LUMEN_C_TRUNCATED] = c_trunc;
   cv[LUMEN_C_MULTI] = c_multi;
   cv[LUMEN_C_MOMENT_LOST] = c_lost;
-  cv[LUMEN_N_COUNT] = (unsigned long long)act;  // the live slots
 #pragma unroll
-  for (int k = 0; k < LUMEN_N_COUNT + 1; ++k) {
+  for (int k = 0; k < LUMEN_N_COUNT; ++k) {
     unsigned long long v = cv[k];
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(FULL, v, o);
     if (lane == 0) sc[k][warp] = v;
   }
   __syncthreads();
-  if (threadIdx.x < LUMEN_N_HEALTH) {
-    double v = sh_health[threadIdx.x];
-    if (v != 0.0) atomicAdd(L.T.health + threadIdx.x, v);
-  } else if (threadIdx.x >= 32 && threadIdx.x < 32 + LUMEN_N_COUNT + 1) {
-    int k = threadIdx.x - 32;
+  for (int k = threadIdx.x; k < LUMEN_N_HEALTH + LUMEN_N_COUNT; k += blockDim.x) {
+    if (k < LUMEN_N_HEALTH) {
+      double v = sh_health[k];
+      if (v != 0.0) atomicAdd(L.T.health + k, v);
+      continue;
+    }
+    const int c = k - LUMEN_N_HEALTH;
     unsigned long long v = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sc[k][w];
-    if (v) atomicAdd(k < LUMEN_N_COUNT ? L.T.counts + k : V.live, v);
-    if (k == LUMEN_C_STEPS && v && L.step_budget > 0) {  // the call's step budget, counted per block
+    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) v += sc[c][w];
+    if (v) atomicAdd(L.T.counts + c, v);
+    if (c == LUMEN_C_STEPS && v && L.step_budget > 0) {  // the call's step budget, counted per block
       unsigned long long used = atomicAdd(L.steps_used, v) + v;
       if (used > (unsigned long long)L.step_budget && atomicExch(L.abort_flag, 1) == 0)
         atomicAdd(L.T.counts + LUMEN_C_ABORTED, 1ull);
@@ -673,22 +797,74 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 }
 
 // The wavefront's rounds (LUMEN_VARIANT_WAVEFRONT): a fill, then query and step kernels, then the drain: the
-// persistent loop resumes every slot still live (one thread a slot) and takes the photons left. A synchronous call
-// reads the live slots back every fourth round and drains once fewer than a 64th of the slots are live (the tail,
-// where a round's launches cost more than its few steps: measured against an 8th, 16th, 32nd, 256th and 1024th); an asynchronous one (LUMEN_F_ASYNC) runs `rounds` rounds
-// without a readback (<= 0: *rpp rounds per photon a slot carries, the scene's estimate from its last synchronous
-// call) and drains. The pool holds up to LUMEN_WAVE_POOL slots (about 350 bytes each with gradients), allocated on the
-// call's stream.
+// persistent loop resumes every slot still live (one thread a slot) and takes the photons left. Each round's query
+// writes its live slots to page-locked host memory as it starts (`pub`), and a synchronous call launches round r once
+// it has seen round r - LUMEN_WAVE_AHEAD's: no round waits for the host, the grids follow the live slots down (they
+// only ever fall), and the drain starts once fewer than a 64th of the slots are live. An asynchronous call
+// (LUMEN_F_ASYNC) runs `rounds` rounds over the whole pool without a readback (<= 0: *rpp rounds per photon a slot
+// carries, the scene's estimate from its last synchronous call) and drains. Against rounds over the whole pool with a
+// readback every fourth (2^24 photons of the tank 45.5 -> 43.6 ms, 1,000,003 5.08 -> 3.83, the ground-wall tank with
+// four tangents 19.7 -> 13.1, the track events 19.9 -> 16.1, the liquid-argon box's 131,072 48 -> 41, the readout tank's
+// 300,007 11.2 -> 9.2); draining at a 256th of the slots, at 2048 or at 64 of them, or looking one or three rounds ahead
+// measured the same within 3 %. The pool holds up to LUMEN_WAVE_POOL slots
+// (about 360 bytes each with gradients), allocated on the call's stream.
 #define LUMEN_WAVE_POOL (1 << 21)
+#define LUMEN_WAVE_AHEAD 2
+
+// threads a block for n live slots: whole blocks of 256 while they fill the chip several times over, fewer where that
+// leaves SMs without one (148 SMs)
+inline int wave_block(unsigned n) { return n >= 148u * 256u * 4u ? 256 : (n >= 148u * 128u * 2u ? 128 : (n >= 148u * 64u ? 64 : 32)); }
+
+// waits for a published round >= `want`; returns its live slots, or -1 where the stream failed
+inline long long wave_seen(volatile unsigned long long* pub, long long want, cudaStream_t stream) {
+  for (long long spin = 0;; ++spin) {
+    const unsigned long long v = *pub;
+    if (v != ~0ull && (long long)(v >> 32) >= want) return (long long)(v & 0xffffffffull);
+    if ((spin & 1023) == 1023) {  // the stream has ended or failed: the last write is there, or never comes
+      const cudaError_t e = cudaStreamQuery(stream);
+      if (e != cudaErrorNotReady) {
+        const unsigned long long w = *pub;
+        if (e == cudaSuccess && w != ~0ull && (long long)(w >> 32) >= want) return (long long)(w & 0xffffffffull);
+        return -1;
+      }
+    }
+  }
+}
+
+// the wavefront's launchers (one instantiation of a kernel in one part of the build)
+template <int EXT, int NAV64>
+int launch_wave_fill(const Launch& L, const Wave& V, cudaStream_t stream) {
+  k_wave_fill<EXT, NAV64><<<V.W / 256, 256, 0, stream>>>(L, V);
+  CK(cudaGetLastError());
+  ++lumen_launches();
+  return 0;
+}
+template <int TORUS, int NAV64>
+int launch_wave_query(const Launch& L, const Wave& V, int grid, int block, cudaStream_t stream) {
+  k_wave_query<TORUS, NAV64><<<grid, block, 0, stream>>>(L, V);
+  CK(cudaGetLastError());
+  ++lumen_launches();
+  return 0;
+}
+template <int G, int BORN, int EXT, int NAV64>
+int launch_wave_step(const Launch& L, const Wave& V, int grid, int block, cudaStream_t stream) {
+  k_wave_step<G, BORN, EXT, NAV64><<<grid, block, 0, stream>>>(L, V);
+  CK(cudaGetLastError());
+  ++lumen_launches();
+  return 0;
+}
+
 template <int G>
-int run_wave(const Launch& L, const Pick& pk, unsigned long long* live, cudaStream_t stream, int slots_log2,
+int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStream_t stream, int slots_log2,
              int async, int rounds, float* rpp) {
   const int64_t pool = slots_log2 >= 16 && slots_log2 <= 23 ? (int64_t)1 << slots_log2 : (int64_t)LUMEN_WAVE_POOL;
   int64_t want = L.n < pool ? L.n : pool;
   int W = (int)((want + 255) / 256 * 256);
-  const size_t nph = sizeof(Photon) / 4, nex = sizeof(WaveExtra) / 4, npre = sizeof(Pre) / 4, nq = sizeof(Query) / 4;
+  const size_t nph = (pk.nav64 ? sizeof(PhotonT<double>) : sizeof(Photon)) / 4, nex = sizeof(WaveExtra) / 4;
+  const size_t npre = (pk.nav64 ? sizeof(PreT<double>) : sizeof(Pre)) / 4;
+  const size_t nq = (pk.nav64 ? sizeof(QueryT<double>) : sizeof(Query)) / 4;
   const size_t ng = G > 0 ? LUMEN_MAX_GRAD : 0;
-  size_t words = (size_t)W * (nph + nex + npre + nq + ng + 1);
+  size_t words = (size_t)W * (nph + nex + npre + nq + ng + 3) + 2;
   uint32_t* buf = nullptr;
   CK(cudaMallocAsync((void**)&buf, words * 4, stream));
   Wave V;
@@ -698,54 +874,79 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* live, cudaStre
   V.pre = V.ex + (size_t)W * nex;
   V.q = V.pre + (size_t)W * npre;
   V.dw = (float*)(V.q + (size_t)W * nq);
-  V.act = (int32_t*)(V.dw + (size_t)W * ng);
-  V.live = live;
-  const int grid = W / 256;
-  CK(cudaMemsetAsync(V.act, 0, (size_t)W * 4, stream));
-  if (pk.born) k_wave_step<G, 1><<<grid, 256, 0, stream>>>(L, V);  // the fill: every slot takes a photon
-  else k_wave_step<G, 0><<<grid, 256, 0, stream>>>(L, V);
-  CK(cudaGetLastError());
-  ++lumen_launches();
+  int32_t* list[2] = {(int32_t*)(V.dw + (size_t)W * ng), (int32_t*)(V.dw + (size_t)W * ng) + W};
+  V.mid = (uint32_t*)(list[1] + W);
+  unsigned* cnt = V.mid + W;  // the two lists' lengths
+  V.in = list[1];
+  V.n_in = cnt + 1;
+  V.out = list[0];
+  V.n_out = cnt;
+  V.pub = nullptr;
+  V.round = 0;
+  if (!async && pub) {
+    *(volatile unsigned long long*)pub = ~0ull;
+    V.pub = pub;
+  }
+  const int ext = pk.clip || pk.groups;
+  int st = pk.nav64 ? launch_wave_fill<1, 1>(L, V, stream)
+                    : (ext ? launch_wave_fill<1, 0>(L, V, stream) : launch_wave_fill<0, 0>(L, V, stream));
+  if (st) return st;
   const long long per_slot = (L.n + W - 1) / W;  // photons a slot carries in turn
   long long cap = -1;                             // rounds of an asynchronous call
   if (async) {
     const float est = rpp && *rpp > 0.0f ? *rpp : 3.0f;
     cap = rounds > 0 ? rounds : (long long)ceilf(est * (float)per_slot);
   }
-  long long r = 0;
-  int drained = 0;
+  long long r = 0, live = L.n < (int64_t)W ? L.n : W;
   for (;; ++r) {
     if (async && r >= cap) break;
-    if (pk.torus) k_wave_query<G, 1><<<grid, 256, 0, stream>>>(L, V);
-    else if (pk.single) k_wave_query<G, 2><<<grid, 256, 0, stream>>>(L, V);
-    else k_wave_query<G, 0><<<grid, 256, 0, stream>>>(L, V);
-    CK(cudaMemsetAsync(V.live, 0, sizeof(unsigned long long), stream));
-    if (pk.born) k_wave_step<G, 1><<<grid, 256, 0, stream>>>(L, V);
-    else k_wave_step<G, 0><<<grid, 256, 0, stream>>>(L, V);
-    CK(cudaGetLastError());
-    lumen_launches() += 2;
-    if (!async && (r & 3) == 3) {
-      unsigned long long h = 0;
-      CK(cudaMemcpyAsync(&h, V.live, sizeof(h), cudaMemcpyDeviceToHost, stream));
-      CK(cudaStreamSynchronize(stream));
-      if (h == 0) break;
-      if (h < (unsigned long long)(W / 64)) {
-        drained = 1;
-        ++r;
-        break;
+    if (!async && r >= LUMEN_WAVE_AHEAD) {
+      live = wave_seen(pub, r - LUMEN_WAVE_AHEAD, stream);
+      if (live < 0) {
+        CK(cudaStreamSynchronize(stream));
+        return set_err(LUMEN_ERR_CUDA, "the wavefront's rounds ended early");
       }
+      if (live < W / 64) break;
     }
+    std::swap(list[0], list[1]);
+    V.in = list[1];
+    V.out = list[0];
+    V.n_in = cnt + (r & 1);
+    V.n_out = cnt + ((r + 1) & 1);
+    V.round = (unsigned)r;
+    const int block = wave_block((unsigned)live), grid = (int)((live + block - 1) / block);
+    if (pk.nav64)
+      st = pk.single ? launch_wave_query<2, 1>(L, V, grid, block, stream)
+                     : (pk.groups ? launch_wave_query<3, 1>(L, V, grid, block, stream)
+                                  : launch_wave_query<1, 1>(L, V, grid, block, stream));
+    else if (pk.groups) st = launch_wave_query<3, 0>(L, V, grid, block, stream);
+    else if (pk.torus) st = launch_wave_query<1, 0>(L, V, grid, block, stream);
+    else if (pk.single) st = launch_wave_query<2, 0>(L, V, grid, block, stream);
+    else st = launch_wave_query<0, 0>(L, V, grid, block, stream);
+    if (st) return st;
+    if (pk.nav64) st = launch_wave_step<G, 1, 1, 1>(L, V, grid, block, stream);
+    else if (pk.born) st = launch_wave_step<G, 1, 1, 0>(L, V, grid, block, stream);
+    else if (ext) st = launch_wave_step<G, 0, 1, 0>(L, V, grid, block, stream);
+    else st = launch_wave_step<G, 0, 0, 0>(L, V, grid, block, stream);
+    if (st) return st;
   }
-  if (async || drained) {  // the persistent loop finishes the live slots and takes the photons left
+  if (live > 0) {  // the persistent loop finishes the live slots and takes the photons left
     Launch LD = L;
     LD.wv_ph = V.ph;
     LD.wv_ex = V.ex;
     LD.wv_dw = V.dw;
-    LD.wv_act = V.act;
+    LD.wv_list = V.out;
+    LD.wv_n = V.n_out;
     LD.wv_W = W;
-    int st = pk.torus ? launch_shape<G, 256, 4, 1>(LD, 0, stream, grid)
-                      : (pk.single ? launch_shape<G, 256, 4, 2>(LD, 0, stream, grid)
-                                   : launch_shape<G, 256, 4, 0>(LD, 0, stream, grid));  // fmt: skip
+    const int grid = (int)(((async ? W : live) + 255) / 256);
+    if (pk.nav64)
+      st = pk.single ? launch_shape<G, 256, 4, 2, 0, 1>(LD, 0, stream, grid)
+                     : (pk.groups ? launch_shape<G, 256, 4, 3, 0, 1>(LD, 0, stream, grid)
+                                  : launch_shape<G, 256, 4, 1, 0, 1>(LD, 0, stream, grid));
+    else if (pk.groups) st = launch_shape<G, 256, 4, 3>(LD, 0, stream, grid);
+    else if (pk.torus) st = launch_shape<G, 256, 4, 1>(LD, 0, stream, grid);
+    else if (pk.single) st = launch_shape<G, 256, 4, 2>(LD, 0, stream, grid);
+    else st = launch_shape<G, 256, 4, 0>(LD, 0, stream, grid);
     if (st) return st;
   }
   if (!async && rpp && per_slot > 0) *rpp = (float)r / (float)per_slot;
@@ -806,6 +1007,24 @@ int launch_event_locate(const DScene& S, const LumenSource& src, int32_t* ev_vol
 #define LUMEN_SHAPES(X) LUMEN_SHAPES_0(X) LUMEN_SHAPES_1(X) LUMEN_SHAPES_2(X) LUMEN_SHAPES_3(X) LUMEN_SHAPES_4(X) \
   LUMEN_SHAPES_5(X) LUMEN_SHAPES_6(X) LUMEN_SHAPES_7(X) LUMEN_SHAPES_8(X) LUMEN_SHAPES_9(X)
 #define LUMEN_SHAPE_DECL(G, B, M, T, A, N) int launch_shape<G, B, M, T, A, N>(const Launch&, int, cudaStream_t, int);
-// part 10: the wavefront's rounds; part 11: the per-photon, query and locate kernels
-#define LUMEN_N_PARTS 12
+// part 11: the per-photon, query and locate kernels; 10 and 12 to 20: the wavefront's (fills EXT, NAV64; queries TORUS,
+// NAV64; steps G, BORN, EXT, NAV64)
+#define LUMEN_WAVE_FILLS(X) X(0, 0) X(1, 0) X(1, 1)
+#define LUMEN_WAVE_QUERIES_10(X) X(2, 0) X(0, 0)
+#define LUMEN_WAVE_QUERIES_12(X) X(1, 0) X(3, 0)
+#define LUMEN_WAVE_QUERIES_13(X) X(2, 1) X(1, 1) X(3, 1)
+#define LUMEN_WAVE_STEPS_14(X) X(0, 0, 0, 0) X(0, 0, 1, 0)
+#define LUMEN_WAVE_STEPS_15(X) X(0, 1, 1, 0)
+#define LUMEN_WAVE_STEPS_16(X) X(0, 1, 1, 1)
+#define LUMEN_WAVE_STEPS_17(X) X(8, 0, 0, 0)
+#define LUMEN_WAVE_STEPS_18(X) X(8, 0, 1, 0)
+#define LUMEN_WAVE_STEPS_19(X) X(8, 1, 1, 0)
+#define LUMEN_WAVE_STEPS_20(X) X(8, 1, 1, 1)
+#define LUMEN_WAVE_QUERIES(X) LUMEN_WAVE_QUERIES_10(X) LUMEN_WAVE_QUERIES_12(X) LUMEN_WAVE_QUERIES_13(X)
+#define LUMEN_WAVE_STEPS(X) LUMEN_WAVE_STEPS_14(X) LUMEN_WAVE_STEPS_15(X) LUMEN_WAVE_STEPS_16(X) \
+  LUMEN_WAVE_STEPS_17(X) LUMEN_WAVE_STEPS_18(X) LUMEN_WAVE_STEPS_19(X) LUMEN_WAVE_STEPS_20(X)
+#define LUMEN_WAVE_FILL_DECL(E, N) int launch_wave_fill<E, N>(const Launch&, const Wave&, cudaStream_t);
+#define LUMEN_WAVE_QUERY_DECL(T, N) int launch_wave_query<T, N>(const Launch&, const Wave&, int, int, cudaStream_t);
+#define LUMEN_WAVE_STEP_DECL(G, B, E, N) int launch_wave_step<G, B, E, N>(const Launch&, const Wave&, int, int, cudaStream_t);
+#define LUMEN_N_PARTS 21
 

@@ -6,6 +6,8 @@
 #error "compile with -DLUMEN_PART=k"
 #endif
 #define LUMEN_INST_SHAPE(G, B, M, T, A, N) template LUMEN_SHAPE_DECL(G, B, M, T, A, N)
+#define LUMEN_INST_QUERY(T, N) template LUMEN_WAVE_QUERY_DECL(T, N)
+#define LUMEN_INST_STEP(G, B, E, N) template LUMEN_WAVE_STEP_DECL(G, B, E, N)
 #if LUMEN_PART == 0
 LUMEN_SHAPES_0(LUMEN_INST_SHAPE)
 #elif LUMEN_PART == 1
@@ -27,12 +29,27 @@ LUMEN_SHAPES_8(LUMEN_INST_SHAPE)
 #elif LUMEN_PART == 9
 LUMEN_SHAPES_9(LUMEN_INST_SHAPE)
 #elif LUMEN_PART == 10
-// the drain's persistent loops are the other parts' instantiations
-#define LUMEN_EXTERN_SHAPE(G, B, M, T, A, N) extern template LUMEN_SHAPE_DECL(G, B, M, T, A, N)
-LUMEN_SHAPES(LUMEN_EXTERN_SHAPE)
-template int run_wave<0>(const Launch&, const Pick&, unsigned long long*, cudaStream_t, int, int, int, float*);
-template int run_wave<LUMEN_MAX_GRAD>(const Launch&, const Pick&, unsigned long long*, cudaStream_t, int, int, int,
-                                      float*);
+#define LUMEN_INST_FILL(E, N) template LUMEN_WAVE_FILL_DECL(E, N)
+LUMEN_WAVE_FILLS(LUMEN_INST_FILL)
+LUMEN_WAVE_QUERIES_10(LUMEN_INST_QUERY)
+#elif LUMEN_PART == 12
+LUMEN_WAVE_QUERIES_12(LUMEN_INST_QUERY)
+#elif LUMEN_PART == 13
+LUMEN_WAVE_QUERIES_13(LUMEN_INST_QUERY)
+#elif LUMEN_PART == 14
+LUMEN_WAVE_STEPS_14(LUMEN_INST_STEP)
+#elif LUMEN_PART == 15
+LUMEN_WAVE_STEPS_15(LUMEN_INST_STEP)
+#elif LUMEN_PART == 16
+LUMEN_WAVE_STEPS_16(LUMEN_INST_STEP)
+#elif LUMEN_PART == 17
+LUMEN_WAVE_STEPS_17(LUMEN_INST_STEP)
+#elif LUMEN_PART == 18
+LUMEN_WAVE_STEPS_18(LUMEN_INST_STEP)
+#elif LUMEN_PART == 19
+LUMEN_WAVE_STEPS_19(LUMEN_INST_STEP)
+#elif LUMEN_PART == 20
+LUMEN_WAVE_STEPS_20(LUMEN_INST_STEP)
 #elif LUMEN_PART == 11
 template int launch_event_locate<0>(const DScene&, const LumenSource&, int32_t*, cudaStream_t);
 template int launch_event_locate<1>(const DScene&, const LumenSource&, int32_t*, cudaStream_t);

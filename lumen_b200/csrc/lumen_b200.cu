@@ -36,9 +36,12 @@ static void begin_call() {
 // the launchers instantiated in the other parts of the build
 #define LUMEN_EXTERN_SHAPE(G, B, M, T, A, N) extern template LUMEN_SHAPE_DECL(G, B, M, T, A, N)
 LUMEN_SHAPES(LUMEN_EXTERN_SHAPE)
-extern template int run_wave<0>(const Launch&, const Pick&, unsigned long long*, cudaStream_t, int, int, int, float*);
-extern template int run_wave<LUMEN_MAX_GRAD>(const Launch&, const Pick&, unsigned long long*, cudaStream_t, int, int,
-                                             int, float*);
+#define LUMEN_EXTERN_FILL(E, N) extern template LUMEN_WAVE_FILL_DECL(E, N)
+LUMEN_WAVE_FILLS(LUMEN_EXTERN_FILL)
+#define LUMEN_EXTERN_QUERY(T, N) extern template LUMEN_WAVE_QUERY_DECL(T, N)
+LUMEN_WAVE_QUERIES(LUMEN_EXTERN_QUERY)
+#define LUMEN_EXTERN_STEP(G, B, E, N) extern template LUMEN_WAVE_STEP_DECL(G, B, E, N)
+LUMEN_WAVE_STEPS(LUMEN_EXTERN_STEP)
 extern template int launch_event_locate<0>(const DScene&, const LumenSource&, int32_t*, cudaStream_t);
 extern template int launch_event_locate<1>(const DScene&, const LumenSource&, int32_t*, cudaStream_t);
 extern template int launch_photons<0>(const Launch&, int32_t*, float*, cudaStream_t);
@@ -621,7 +624,9 @@ static int check_cells(const Tally& T) {
 
 static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* cot, int n_events_cot, double* grads,
                      cudaStream_t stream, int variant = 0, int bps = 0, int async = 0, int slots_log2 = 0,
-                     int rounds = 0, float* rpp = nullptr) {
+                     int rounds = 0, const LumenScene* sc = nullptr) {
+  float* rpp = sc ? &sc->wave_rpp : nullptr;
+  PubLease pub(sc);
   Tally& T = L.T;
   T.E = out ? (out->n_events > 0 ? out->n_events : 1) : (n_events_cot > 0 ? n_events_cot : 1);
   T.S_ = L.R.S.n_sensor > 0 ? L.R.S.n_sensor : 1;
@@ -632,24 +637,24 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
     L.truth = out->truth;
     if (variant == LUMEN_VARIANT_WAVEFRONT) variant = 0;
   }
-  if ((pk.nav64 || pk.clip) && variant == LUMEN_VARIANT_WAVEFRONT) variant = 0;  // the wavefront's slots hold float32 positions
+  if (variant == LUMEN_VARIANT_WAVEFRONT && !async)
+    if (int st = pub.take()) return st;
   T.grads = grads;
-  // scratch: the photon counter, the abort flag, the steps used, the wavefront's live slots and the record count (one
-  // small allocation per call)
+  // scratch: the photon counter, the abort flag, the steps used and the record count (one small allocation per call)
   const int groups = out && out->n_groups > 0;
   int st0 = 0;
   if (groups && (st0 = check_groups(L.R.S.n_sensor, out))) return st0;
   if ((st0 = check_cells(T))) return st0;
   unsigned long long* scratch = nullptr;
-  CK(cudaMallocAsync((void**)&scratch, 5 * sizeof(unsigned long long), stream));
-  CK(cudaMemsetAsync(scratch, 0, 5 * sizeof(unsigned long long), stream));
+  CK(cudaMallocAsync((void**)&scratch, 4 * sizeof(unsigned long long), stream));
+  CK(cudaMemsetAsync(scratch, 0, 4 * sizeof(unsigned long long), stream));
   L.next = scratch;
   L.abort_flag = (int*)(scratch + 1);
   L.steps_used = scratch + 2;
   if (groups) {
     L.R.rec = (uint32_t*)out->records;
     L.R.rec_cap = out->rec_capacity;
-    L.R.rec_n = scratch + 4;
+    L.R.rec_n = scratch + 3;
   }
   // adjoint calls with no tallies of their own accumulate health and counts into the scratch's tail
   double* dummy = nullptr;
@@ -700,11 +705,11 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
         L2.T.counts = (unsigned long long*)(dummy + LUMEN_N_HEALTH);
       }
       st = variant == LUMEN_VARIANT_WAVEFRONT
-               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, scratch + 3, stream, slots_log2, async, rounds, rpp)
+               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub.p, stream, slots_log2, async, rounds, rpp)
                : launch_trace<LUMEN_MAX_GRAD>(L2, pk, variant, bps, stream);
       if (st) return st;
     } else {
-      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, scratch + 3, stream, slots_log2, async, rounds, rpp)
+      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub.p, stream, slots_log2, async, rounds, rpp)
                                               : launch_trace<0>(L, pk, variant, bps, stream);
       if (st) return st;
     }
@@ -723,7 +728,7 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
   int flag = 0;
   unsigned long long n_rec = 0;
   CK(cudaMemcpyAsync(&flag, L.abort_flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  CK(cudaMemcpyAsync(&n_rec, scratch + 4, sizeof(n_rec), cudaMemcpyDeviceToHost, stream));
+  CK(cudaMemcpyAsync(&n_rec, scratch + 3, sizeof(n_rec), cudaMemcpyDeviceToHost, stream));
   CK(cudaFreeAsync(scratch, stream));
   if (dummy) CK(cudaFreeAsync(dummy, stream));
   CK(cudaStreamSynchronize(stream));
@@ -1018,7 +1023,7 @@ int32_t lumen_b200_scene_create(const LumenSceneDesc* d, LumenScene** out) {
   }
   sc->tab.assign(d->tab, d->tab + 2 * (size_t)d->n_tab);
   sc->has_torus = d->n_mesh > 0 || d->n_group > 0;  // the extended instantiation: tori, meshes, frame groups
-  sc->clip = d->n_group > 0;  // the extended locate (frame groups, protrusion clips): no wavefront (its fill's locate)
+  sc->clip = d->n_group > 0;  // the extended locate: frame groups, protrusion clips
   sc->groups = d->n_group > 0;
   for (int l = 0; l < d->n_leaf; ++l) sc->has_torus = sc->has_torus || d->leaf_i[(size_t)l * LUMEN_LEAF_I] == 2;
   for (int v = 0; v < d->n_vol && !sc->clip; ++v) {  // a protrusion clip: the extended instantiation
@@ -1100,6 +1105,7 @@ int32_t lumen_b200_adjoint(const LumenScene* sc, const LumenRows* rows, const Lu
                            uint32_t key1, int64_t first_id, int64_t n, const LumenControls* c,
                            const double* cotangent, int32_t n_events, double* grads, void* stream) {
   begin_call();
+  for (unsigned long long* p : sc->pub_free) cudaFreeHost(p);
   if (!cotangent || !grads) return set_err(LUMEN_ERR_ARG, "adjoint: cotangent and grads are required");
   if (!c || c->n_grad <= 0) return set_err(LUMEN_ERR_ARG, "adjoint: no gradient parameters");
   Launch L;
@@ -1108,7 +1114,7 @@ int32_t lumen_b200_adjoint(const LumenScene* sc, const LumenRows* rows, const Lu
   if (st) return st;
   if (pk.analog) return set_err(LUMEN_ERR_ARG, "the adjoint replays no truth rows");
   return run_trace(L, pk, nullptr, cotangent, n_events, grads, (cudaStream_t)stream, c->variant, c->blocks_per_sm,
-                   c->flags & LUMEN_F_ASYNC, c->wave_slots_log2, c->wave_rounds, &sc->wave_rpp);
+                   c->flags & LUMEN_F_ASYNC, c->wave_slots_log2, c->wave_rounds, sc);
 }
 
 int32_t lumen_b200_trace_photons(const LumenScene* sc, const LumenRows* rows, const LumenSource* source,

@@ -20,7 +20,7 @@ FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-li
          "-prec-div=true", "-prec-sqrt=true", "-ftz=false", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC"]  # fmt: skip
 LINK = ["-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC"]
 PART = os.path.join(HERE, "csrc", "k_part.cu")
-N_PARTS = 12  # LUMEN_N_PARTS in csrc/engine.cuh: the kernel instantiations' parts, compiled in parallel
+N_PARTS = 21  # LUMEN_N_PARTS in csrc/engine.cuh: the kernel instantiations' parts, compiled in parallel
 OBJ = os.path.join(HERE, "_build")
 
 
