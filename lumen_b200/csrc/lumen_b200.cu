@@ -64,6 +64,31 @@ __global__ void k_moment_flush(Tally T) {
   }
 }
 
+// A run's results from its tallies, in place (lumen_b200_finish): bandwidth-bound on the cells, one thread a cell, in
+// place of the two dozen element-wise launches and the host passes that made them before. Each operation is the one
+// the host's float64 would make (no contraction), so the results are the same bit for bit.
+__global__ void __launch_bounds__(256) k_finish(Tally T, const int64_t* ev_first, int64_t samples, double* nonfinite) {
+  const size_t cells = (size_t)T.E * T.S_, step = (size_t)gridDim.x * blockDim.x;
+  const size_t k0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long bad = 0;
+  for (size_t k = k0; k < cells; k += step) {
+    const double x = T.arrival[k], xt = T.arrival_t[k], x2 = T.arrival2[k];
+    bad += !isfinite(x) + !isfinite(xt) + !isfinite(x2);
+    const size_t e = k / T.S_;
+    const double n = (double)(ev_first ? ev_first[e + 1] - ev_first[e] : samples);
+    double v = x2 - x * x / (n > 1.0 ? n : 1.0);
+    v = v < 0.0 ? 0.0 : v;
+    T.arrival2[k] = sqrt(n / (n - 1.0 > 1.0 ? n - 1.0 : 1.0) * v);
+    T.arrival_t[k] = x > 0.0 ? xt / x : __longlong_as_double(0x7ff8000000000000ll);
+  }
+  if (T.hist)
+    for (size_t k = k0; k < cells * T.nb; k += step) bad += !isfinite(T.hist[k]);
+  if (T.jac)
+    for (size_t k = k0; k < cells * T.P; k += step) bad += !isfinite(T.jac[k]);
+  for (int o = 16; o > 0; o >>= 1) bad += __shfl_down_sync(0xffffffffu, bad, o);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(nonfinite, (double)bad);
+}
+
 // ------------------------------------------------------------------------------------------- host helpers
 static int upload_raw(LumenScene* sc, const void* h, size_t bytes, void** out) {
   *out = nullptr;
@@ -1080,6 +1105,7 @@ int32_t lumen_b200_scene_destroy(LumenScene* sc) {
   begin_call();
   if (!sc) return 0;
   for (void* p : sc->allocs) cudaFree(p);
+  for (unsigned long long* p : sc->pub_free) cudaFreeHost(p);
   delete sc;
   return 0;
 }
@@ -1098,14 +1124,13 @@ int32_t lumen_b200_trace(const LumenScene* sc, const LumenRows* rows, const Lume
   int st = fill_launch(sc, rows, source, key0, key1, first_id, n, c, L, pk);
   if (st) return st;
   return run_trace(L, pk, out, nullptr, 0, nullptr, (cudaStream_t)stream, c->variant, c->blocks_per_sm,
-                   c->flags & LUMEN_F_ASYNC, c->wave_slots_log2, c->wave_rounds, &sc->wave_rpp);
+                   c->flags & LUMEN_F_ASYNC, c->wave_slots_log2, c->wave_rounds, sc);
 }
 
 int32_t lumen_b200_adjoint(const LumenScene* sc, const LumenRows* rows, const LumenSource* source, uint32_t key0,
                            uint32_t key1, int64_t first_id, int64_t n, const LumenControls* c,
                            const double* cotangent, int32_t n_events, double* grads, void* stream) {
   begin_call();
-  for (unsigned long long* p : sc->pub_free) cudaFreeHost(p);
   if (!cotangent || !grads) return set_err(LUMEN_ERR_ARG, "adjoint: cotangent and grads are required");
   if (!c || c->n_grad <= 0) return set_err(LUMEN_ERR_ARG, "adjoint: no gradient parameters");
   Launch L;
@@ -1115,6 +1140,33 @@ int32_t lumen_b200_adjoint(const LumenScene* sc, const LumenRows* rows, const Lu
   if (pk.analog) return set_err(LUMEN_ERR_ARG, "the adjoint replays no truth rows");
   return run_trace(L, pk, nullptr, cotangent, n_events, grads, (cudaStream_t)stream, c->variant, c->blocks_per_sm,
                    c->flags & LUMEN_F_ASYNC, c->wave_slots_log2, c->wave_rounds, sc);
+}
+
+int32_t lumen_b200_finish(LumenTallies* t, int32_t n_sensor, int32_t n_grad, const int64_t* ev_first, int64_t samples,
+                          double* nonfinite, void* stream) {
+  begin_call();
+  if (!t || !t->arrival || !t->arrival_t || !t->arrival2 || !nonfinite)
+    return set_err(LUMEN_ERR_ARG, "finish: a required array is null");
+  if (n_grad < 0 || n_grad > LUMEN_MAX_GRAD || (n_grad > 0 && !t->jac) || (t->hist && t->n_bins <= 0))
+    return set_err(LUMEN_ERR_ARG, "finish: a bad Jacobian or histogram");
+  Tally T;
+  memset(&T, 0, sizeof(T));
+  T.E = t->n_events > 0 ? t->n_events : 1;
+  T.S_ = n_sensor > 0 ? n_sensor : 1;
+  T.P = n_grad;
+  T.nb = t->hist ? t->n_bins : 0;
+  T.arrival = t->arrival;
+  T.arrival_t = t->arrival_t;
+  T.arrival2 = t->arrival2;
+  T.hist = t->hist;
+  T.jac = n_grad > 0 ? t->jac : nullptr;
+  const size_t cells = (size_t)T.E * T.S_, most = cells * (size_t)std::max(1, std::max(T.nb, T.P));
+  const size_t want = (most + 255) / 256;
+  CK(cudaMemsetAsync(nonfinite, 0, sizeof(double), (cudaStream_t)stream));
+  k_finish<<<(unsigned)std::min<size_t>(want, 148 * 8), 256, 0, (cudaStream_t)stream>>>(T, ev_first, samples, nonfinite);
+  CK(cudaGetLastError());
+  ++lumen_launches();
+  return 0;
 }
 
 int32_t lumen_b200_trace_photons(const LumenScene* sc, const LumenRows* rows, const LumenSource* source,

@@ -118,7 +118,7 @@ def simulate_sharded(det, source, params=None, *, samples=None, seed=0, referenc
     else:
         T = tracer(first, n, key, c, DeviceTallies(det.n_sensor, n_ev, nb, t0, tw, len(gt), "cpu"))
     all_reduce_tallies(T, group)
-    light = api._light(det, T, n_ev, total, seed, gnames, (nb, t0, tw), source)
+    light = api._light(det, T, n_ev, total, seed, gnames, (nb, t0, tw), source, eng=None if tracer else eng)
     light.provenance.update(world=world, rank=rank, shard=(first, n))
     return light
 

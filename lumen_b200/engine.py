@@ -8,6 +8,7 @@ engine raises.
 from __future__ import annotations
 
 import ctypes
+import math
 
 import numpy as np
 import torch
@@ -36,12 +37,20 @@ class DeviceTallies:
 
     def __init__(self, n_sensor, n_events=1, n_bins=0, bin0=0.0, bin_w=1.0, n_grad=0, device="cuda"):
         S, E = max(n_sensor, 1), max(n_events, 1)
-        z = lambda *s: torch.zeros(*s, dtype=torch.float64, device=device)  # noqa: E731
-        self.arrival, self.arrival_t, self.arrival2 = z(E, S), z(E, S), z(E, S)
-        self.hist = z(E, S, n_bins) if n_bins else None
-        self.jac = z(E, S, n_grad) if n_grad else None
-        self.health = z(A.N_HEALTH)
-        self.counts = torch.zeros(A.N_COUNT, dtype=torch.int64, device=device)
+        # one buffer, zeroed at once and read back at once: each tally a view of it, the last word lumen_b200_finish's
+        # count of cells that are not finite
+        shapes = {"arrival": (E, S), "arrival_t": (E, S), "arrival2": (E, S), "hist": (E, S, n_bins) if n_bins else None,
+                  "jac": (E, S, n_grad) if n_grad else None, "health": (A.N_HEALTH,), "counts": (A.N_COUNT,),
+                  "nonfinite": (1,)}  # fmt: skip
+        sizes = {k: math.prod(v) for k, v in shapes.items() if v is not None}
+        self.flat = torch.zeros(sum(sizes.values()), dtype=torch.float64, device=device)
+        self.at, o = {}, 0
+        for k, v in shapes.items():
+            setattr(self, k, self.flat[o:o + sizes[k]].view(v) if v is not None else None)
+            if v is not None:
+                self.at[k] = (o, v)
+                o += sizes[k]
+        self.counts = self.counts.view(torch.int64)
         t = A.LumenTallies()
         t.n_events, t.n_bins, t.bin0, t.bin_w = E, n_bins, bin0, bin_w
         t.arrival, t.arrival_t, t.arrival2 = _f64p(self.arrival), _f64p(self.arrival_t), _f64p(self.arrival2)
@@ -65,9 +74,7 @@ class DeviceTallies:
         return self
 
     def zero_(self):
-        for v in (self.arrival, self.arrival_t, self.arrival2, self.hist, self.jac, self.health, self.counts):
-            if v is not None:
-                v.zero_()
+        self.flat.zero_()
         if getattr(self, "groups", None) is not None:
             self.groups.zero_()
         return self
@@ -78,9 +85,14 @@ class DeviceSource:
 
     def __init__(self, src, samples, device="cuda", det=None):
         a = src.arrays(samples, det)
-        self.ev_f = torch.as_tensor(np.ascontiguousarray(a["ev_f"], np.float32), device=device)
-        self.ev_first = torch.as_tensor(np.ascontiguousarray(a["ev_first"], np.int64), device=device)
-        self.ev_w = torch.as_tensor(np.ascontiguousarray(a["ev_w"], np.float32), device=device)
+        # the three arrays in one copy: int64, then the float32 ones
+        self.first = np.ascontiguousarray(a["ev_first"], np.int64)
+        parts = [self.first, np.ascontiguousarray(a["ev_f"], np.float32), np.ascontiguousarray(a["ev_w"], np.float32)]
+        dev = torch.from_numpy(np.concatenate([p.reshape(-1).view(np.uint8) for p in parts])).to(device)
+        k = [p.nbytes for p in parts]
+        self.ev_first = dev[:k[0]].view(torch.int64)
+        self.ev_f = dev[k[0]:k[0] + k[1]].view(torch.float32).view(parts[1].shape)
+        self.ev_w = dev[k[0] + k[1]:].view(torch.float32)
         s = A.LumenSource()
         s.kind, s.n_events = a["kind"], len(a["ev_w"])
         s.ev_f, s.ev_first, s.ev_w = _f32p(self.ev_f), _i64p(self.ev_first), _f32p(self.ev_w)
@@ -183,6 +195,15 @@ class Engine:
             A.check(self.lib.lumen_b200_adjoint(self.h, rw, src, key[0], key[1], first_id, n, ctypes.byref(c),
                                                 _f64p(cot), n_ev, _f64p(grads), self._stream(stream)))  # fmt: skip
         return grads
+
+    def finish(self, T, samples, ev_first=None):
+        """Turn the tallies T in place into a run's results (``lumen_b200_finish``): ``arrival2`` each cell's Monte Carlo
+        error, ``arrival_t`` its mean arrival time, ``nonfinite`` the count of output cells that are not finite; an
+        event's photons are ``samples``, or the differences of ``ev_first`` (int64, on the device)."""  # noqa: D205
+        n_grad = 0 if T.jac is None else T.jac.shape[-1]
+        with torch.cuda.device(self.device):
+            A.check(self.lib.lumen_b200_finish(ctypes.byref(T.c), T.arrival.shape[1], n_grad, _i64p(ev_first),
+                                               int(samples), _f64p(T.nonfinite), self._stream(None)))  # fmt: skip
 
     def trace_photons(self, key, n, *, source=None, rows=None, first_id=0, controls=None):
         c = controls or A.controls()
