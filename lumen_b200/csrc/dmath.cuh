@@ -21,13 +21,23 @@
 // surface kernel, the media and the navigator's helpers called (their frames and argument copies were local memory)
 #define L_CALL static __device__ __noinline__
 
+// loops whose count is the call's or the data's stay rolled: the compiler's copies by four were most of a kernel's code,
+// and the kernels wait on instruction fetch (the step kernel with tangents 10 stalls an issue on it). With the settle's
+// solids read in the scene's own instantiation (dnav.cuh d_ray_holds), same box, ms: the tank's 2^24 photons 43.1 -> 40.0,
+// the ground-wall tank with four tangents 12.6 -> 11.3, the track events 14.1 -> 13.3, the liquid-argon box 25.0 -> 23.9,
+// the readout tank 8.8 -> 8.1, the solids box 9.6 -> 8.6, the float64 panel 4.2 -> 4.0
+#define L_ROLL _Pragma("unroll 1")
+// the elementary functions: inlined, or one copy a kernel where the part says so (k_part.cu)
+#ifndef L_MATH
+#define L_MATH L_DEV
+#endif
 namespace lb {
 
 L_DEV float bits_f(uint32_t u) { return __uint_as_float(u); }
 L_DEV uint32_t f_bits(float f) { return __float_as_uint(f); }
 L_DEV float pow2i(int k) { return bits_f((uint32_t)(k + 127) << 23); }
 
-L_DEV float l_exp(float x) {
+L_MATH float l_exp(float x) {
   if (!(x == x)) return x;
   if (x > 88.72283935546875f) return __int_as_float(0x7f800000);
   if (x < -103.972084045410f) return 0.0f;
@@ -51,7 +61,7 @@ L_DEV float l_exp(float x) {
   return p * pow2i(k);
 }
 
-L_DEV float l_log(float x) {
+L_MATH float l_log(float x) {
   if (!(x > 0.0f)) return x == 0.0f ? __int_as_float(0xff800000) : __int_as_float(0x7fc00000);
   if (x == __int_as_float(0x7f800000)) return x;
   int adj = 0;
@@ -99,7 +109,7 @@ L_DEV void l_quadrant(int q, float s, float c, float* so, float* co) {
   }
 }
 
-L_DEV float2 l_sincos2pi_v(float u) {
+L_MATH float2 l_sincos2pi_v(float u) {
   float v = 4.0f * u;
   float q = floorf(v + 0.5f);
   float f = v - q;
@@ -110,7 +120,7 @@ L_DEV float2 l_sincos2pi_v(float u) {
   return make_float2(s, c);
 }
 
-L_DEV float2 l_sincos_v(float x) {
+L_MATH float2 l_sincos_v(float x) {
   const float TWO_OVER_PI = 0.636619772367581343076f;
   const float P1 = 1.5703125f;
   const float P2 = 4.83512878417968750000e-4f;
@@ -147,7 +157,7 @@ L_DEV float l_asin_small(float x) {
   return fmaf(x * z, p, x);
 }
 
-L_DEV float l_acos(float x) {
+L_MATH float l_acos(float x) {
   const float PI = 3.14159265358979323846f;
   const float PIO2 = 1.57079632679489661923f;
   if (x > 1.0f) x = 1.0f;
@@ -166,7 +176,7 @@ L_DEV float l_asin(float v) {
 }
 
 // atan2 from asin / acos on the octant where each is well conditioned
-L_DEV float l_atan2(float y, float x) {
+L_MATH float l_atan2(float y, float x) {
   const float PI = 3.14159265358979323846f;
   float r = sqrtf(x * x + y * y);
   if (r == 0.0f) return 0.0f;
@@ -181,7 +191,7 @@ L_DEV float l_atan2(float y, float x) {
 }
 
 // the cube root: exp(log|x| / 3) and one Newton step on y^3 = |x|
-L_DEV float l_cbrt(float x) {
+L_MATH float l_cbrt(float x) {
   if (x == 0.0f) return 0.0f;
   float a = x < 0.0f ? -x : x;
   float y = l_exp(l_log(a) * 0.333333343267440796f);
@@ -206,7 +216,7 @@ L_DEV double l_cbrt64(double x) {
   return x < 0.0 ? -y : y;
 }
 
-L_DEV float l_erfinv(float x) {
+L_MATH float l_erfinv(float x) {
   float w = -l_log((1.0f - x) * (1.0f + x));
   float p;
   if (w < 5.0f) {

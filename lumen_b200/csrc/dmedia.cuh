@@ -92,6 +92,7 @@ struct DSpec {
 L_DEV DSpec d_spec(const float* e, const float* s, int k, int cover) {
   DSpec p;
   p.e = e; p.s = s; p.k = k; p.tot = 0.0f; p.Z = 0.0f;
+  L_ROLL
   for (int j = 0; j + 1 < k; ++j) {
     float h = __ldg(e + j + 1) - __ldg(e + j);
     float m = 0.5f * (__ldg(s + j + 1) + __ldg(s + j)) * h;
@@ -119,6 +120,7 @@ L_DEV float d_spec_c_next(const DSpec& p, int j, float c_j, float* mass_acc) {
 L_DEV float d_spec_invert(const DSpec& p, float r) {
   int n = p.k - 1, kk = 0;
   float c = 0.0f, ck = 0.0f, acc = 0.0f;
+  L_ROLL
   for (int j = 0; j < n; ++j) {
     if (c <= r) { kk = j; ck = c; }
     if (j + 1 < n) c = d_spec_c_next(p, j, c, &acc);
@@ -131,6 +133,7 @@ L_DEV float d_spec_invert(const DSpec& p, float r) {
 L_DEV float d_spec_cumulative(const DSpec& p, float E) {
   int n = p.k - 1, kk = 0;
   float c = 0.0f, ck = 0.0f, acc = 0.0f;
+  L_ROLL
   for (int j = 0; j < n; ++j) {
     if (__ldg(p.e + j) <= E) { kk = j; ck = c; }
     if (j + 1 < n) c = d_spec_c_next(p, j, c, &acc);
@@ -145,6 +148,7 @@ L_DEV float d_spec_cumulative(const DSpec& p, float E) {
 L_DEV float d_spec_density(const float* e, const float* s, int k, int cover, float E) {
   if (!(E >= __ldg(e) && E <= __ldg(e + k - 1))) return 0.0f;
   float tot = 0.0f, Z = 0.0f;
+  L_ROLL
   for (int j = 0; j + 1 < k; ++j) {
     float sj = __ldg(s + j), sj1 = __ldg(s + j + 1), h = __ldg(e + j + 1) - __ldg(e + j);
     float t = (sj1 + sj) * h;
@@ -152,6 +156,7 @@ L_DEV float d_spec_density(const float* e, const float* s, int k, int cover, flo
     if (sj1 + sj <= 0.0f && h > 0.0f) Z = Z + h;
   }
   int i = 0;
+  L_ROLL
   for (int j = 0; j < k; ++j)
     if (__ldg(e + j) <= E) i = j;
   i = i > k - 2 ? k - 2 : i;
@@ -206,6 +211,7 @@ L_DEV void d_bulk_other(const DScene& S, const float* __restrict__ live, const f
   const int32_t* m = S.med_i + (size_t)mi * LUMEN_MED_I;
   float E = D_HC / lam;
   b.rlw = 1.0f; b.y_w = 1.0f; b.y_r = 1.0f; b.delay = 0.0f; b.lam = lam;
+  L_ROLL
   for (int p = 0; p < P; ++p) { b.dlob[p] = 0.0f; b.dyld[p] = 0.0f; }
   float r3 = uniform(vkey, 3), r4 = uniform(vkey, 4);
   if (cs == 1) {
@@ -226,6 +232,7 @@ L_DEV void d_bulk_other(const DScene& S, const float* __restrict__ live, const f
     float dl[3];
     float lp = d_mie_logpdf(pl[0], pl[1], pl[2], wi, b.d, dl);
     if (!shared || pr[2] != r0) b.rlw = l_exp(lp - d_mie_logpdf(pr[0], pr[1], pr[2], wi, b.d, nullptr));
+    L_ROLL
     for (int p = 0; p < P; ++p)
       for (int k = 0; k < 3; ++k)
         if (tg[k] == gt[p]) b.dlob[p] = b.dlob[p] + dl[k];
@@ -246,6 +253,7 @@ L_DEV void d_bulk_other(const DScene& S, const float* __restrict__ live, const f
     b.y_r = em.w_r;
     b.delay = em.delay;
     b.lam = em.lam;
+    L_ROLL
     for (int p = 0; p < P; ++p)
       if (ty == gt[p]) b.dyld[p] = em.dyield;
   }

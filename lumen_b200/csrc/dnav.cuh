@@ -205,8 +205,10 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   NF p1 = d_min(d_max(s_v - w, s_lo), s_hi), p2 = d_min(d_max(s_v + w, s_lo), s_hi);
   // the extrema: a minimum on [s_lo, p1] (g' increasing), the maximum on [p1, p2], a minimum on [p2, s_hi]
   NF el[3] = {s_lo, p1, p2}, eh[3] = {p1, p2, s_hi}, e[3];
+  L_ROLL
   for (int k = 0; k < 3; ++k) {
     NF l = el[k], h = eh[k];
+    L_ROLL
     for (int it = 0; it < N_BISECT; ++it) {
       NF mid = 0.5f * (l + h);
       const int closed = mid == l || mid == h;
@@ -222,6 +224,7 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
   const NF knots[7] = {s_lo, e[0], p1, e[1], p2, e[2], s_hi};
   NF t[6];
   int in_k = d_torus_g(R, r, oc, dd, s_lo) <= 0.0f;  // membership at the piece's left end
+  L_ROLL
   for (int k = 0; k < 6; ++k) {
     NF xl = knots[k], xr = knots[k + 1];
     const int inl = in_k, inr = d_torus_g(R, r, oc, dd, xr) <= 0.0f;
@@ -229,6 +232,7 @@ L_CALL void d_torus_set(NF R, NF r, const NF* od, const NF* dd, NF* lo, NF* hi) 
     t[k] = inf;
     if (!(inl != inr && xr > xl)) continue;
     NF l = xl, h = xr;
+    L_ROLL
     for (int it = 0; it < N_BISECT; ++it) {
       NF mid = 0.5f * (l + h);
       const int closed = mid == l || mid == h;
@@ -291,6 +295,7 @@ L_DEV Iv d_leaf_iv(const DScene& S, int g, const NF* o, const NF* d) {
   NF t0p = -inf, t1p = inf;
   int f0p = -1, f1p = -1, ep = 0;
   int p0 = __ldg(li + 1), np_ = __ldg(li + 2);
+  L_ROLL
   for (int k = 0; k < np_; ++k) {
     const NF* pl = NAV_PLANE(S) + (size_t)(p0 + k) * LUMEN_PLANE_F;
     NF n0 = __ldg(pl), n1 = __ldg(pl + 1), n2 = __ldg(pl + 2), h = __ldg(pl + 3);
@@ -323,6 +328,7 @@ L_DEV int d_inside_leaf(const DScene& S, int g, const NF* x) {
   NF y[3] = {x[0] - __ldg(lf + 3), x[1] - __ldg(lf + 4), x[2] - __ldg(lf + 5)};
   int pl = 1;
   int p0 = __ldg(li + 1), np_ = __ldg(li + 2);
+  L_ROLL
   for (int k = 0; k < np_; ++k) {
     const NF* p = NAV_PLANE(S) + (size_t)(p0 + k) * LUMEN_PLANE_F;
     pl = pl && (__ldg(p) * xl[0] + __ldg(p + 1) * xl[1] + __ldg(p + 2) * xl[2] <= __ldg(p + 3));
@@ -348,6 +354,7 @@ L_DEV int d_inside_kind(const DScene& S, int kind, const NF* x) {
   const int32_t* k = S.kind_i + (size_t)kind * LUMEN_KIND_I;
   const int l0 = __ldg(k), nl = __ldg(k + 1);
   unsigned m = 0;
+  L_ROLL
   for (int l = 0; l < nl; ++l) m |= (unsigned)d_inside_leaf(S, l0 + l, x) << l;
   return d_bool(S, kind, m);
 }
@@ -367,7 +374,6 @@ struct ScanT {
   NF on_tend, hend;
 };
 
-using Scan = ScanT<LUMEN_MAX_LEAVES>;
 
 template <int NLMAX>
 L_DEV NF d_scan_band(const ScanT<NLMAX>& s, NF t) { return d_band(s.xa + n_abs(t)); }
@@ -382,6 +388,7 @@ L_DEV int d_mem_at(const DScene& S, const ScanT<NLMAX>& s, NF t, int use_on) {
     return m;
   }
   unsigned mask = 0;
+  L_ROLL
   for (int l = 0; l < s.nl; ++l) {
     const Iv& v = s.iv[l];
     int m = (v.lo0 <= t && t < v.hi0) || (v.lo1 <= t && t < v.hi1);
@@ -400,6 +407,7 @@ L_DEV void d_scan_init(const DScene& S, ScanT<NLMAX>& s, int kind, const NF* o, 
   const int32_t* k = S.kind_i + (size_t)kind * LUMEN_KIND_I;
   s.nl = NLMAX == 1 ? 1 : __ldg(k + 1);
   int l0 = __ldg(k);
+  L_ROLL
   for (int l = 0; l < (NLMAX == 1 ? 1 : s.nl); ++l) {
     if ((TORUS & 1) && __ldg(S.leaf_i + (size_t)(l0 + l) * LUMEN_LEAF_I) == 2)
       s.iv[l] = d_torus_iv(NAV_LEAF(S) + (size_t)(l0 + l) * LUMEN_LEAF_F, NF3{o[0], o[1], o[2]},
@@ -423,6 +431,7 @@ template <int NLMAX>
 L_DEV void d_nearest(const ScanT<NLMAX>& s, NF t_cur, NF* e1o, int* lbo, int* fco, int* eko) {
   NF e1 = N_BIG;
   int lb = -1, jb = 0;
+  L_ROLL
   for (int l = 0; l < (NLMAX == 1 ? 1 : s.nl); ++l) {
     const Iv& v = s.iv[l];
     const int skip = s.has_skip && l == s.skip_leaf;
@@ -447,6 +456,7 @@ L_DEV Fc d_first_change(const DScene& S, ScanT<NLMAX>& s, NF t0) {
   int done = 0, now = 0, lb_h = -1, fc_h = -1, now0 = 0, it = 0;
   First fs = {0, N_HUGE, 0, -1, -1};
   s.hend = s.has_on ? s.on_tend : -N_HUGE;
+  L_ROLL
   while (!done && t_cur < N_HUGE && it < D_MAX_SCAN_PER_LEAF * s.nl + D_MAX_SCAN_EXTRA) {
     int first = it == 0;
     NF e; int lb, fc, ek;
@@ -576,12 +586,13 @@ L_DEV int d_holds_point(const DScene& S, int i, const NF* x) {
   d_to_local_pt(S, i, x, xl);
   return d_inside_kind(S, vI(S, i, LUMEN_VI_KIND), xl);
 }
+template <int TORUS>
 L_DEV int d_ray_holds(const DScene& S, int i, const NF* od, const NF* dd, NF t) {
   NF ol[3], dl[3];
   d_to_local_pt(S, i, od, ol);
   d_to_local_dir(S, i, dd, dl);
-  Scan s;
-  d_scan_init<1>(S, s, vI(S, i, LUMEN_VI_KIND), ol, dl, N_HUGE);
+  ScanT<TORUS == 2 ? 1 : LUMEN_MAX_LEAVES> s;
+  d_scan_init<TORUS>(S, s, vI(S, i, LUMEN_VI_KIND), ol, dl, N_HUGE);
   return d_mem_at(S, s, t, 0);
 }
 L_DEV int d_level_wins(const DScene& S, int item, int found, int excl) {
@@ -593,6 +604,7 @@ template <class F>
 L_DEV void d_point_scan(const DScene& S, int v, const NF* x, NF pad, F visit) {
   int n0 = vI(S, v, LUMEN_VI_NODE0), n1 = vI(S, v, LUMEN_VI_NODE1);
   int node = n0;
+  L_ROLL
   while (node < n1) {
     const NF* nf = NAV_NODE(S) + (size_t)node * LUMEN_NODE_F;
     int inside = (__ldg(nf) - pad <= x[0] && x[0] <= __ldg(nf + 3) + pad) &&
@@ -602,6 +614,7 @@ L_DEV void d_point_scan(const DScene& S, int v, const NF* x, NF pad, F visit) {
     int cnt = __ldg(ni + 1);
     if (inside && cnt > 0) {
       int st = __ldg(ni + 2);
+      L_ROLL
       for (int k = 0; k < cnt; ++k) visit(__ldg(S.items + st + k));
     }
     node = (inside && cnt == 0) ? node + 1 : __ldg(ni);
@@ -622,6 +635,7 @@ L_DEV void d_point_scan_x(const DScene& S, int v, const NF* x, NF pad, F visit) 
   NF xs[3] = {x[0], x[1], x[2]};
   for (int guard = 0; guard <= LUMEN_MAX_GROUPS_PER_VOLUME; ++guard) {
     int node = n0;
+    L_ROLL
     while (node < n1) {
       const NF* nf = NAV_NODE(S) + (size_t)node * LUMEN_NODE_F;
       int inside = (__ldg(nf) - pad <= xs[0] && xs[0] <= __ldg(nf + 3) + pad) &&
@@ -631,6 +645,7 @@ L_DEV void d_point_scan_x(const DScene& S, int v, const NF* x, NF pad, F visit) 
       int cnt = __ldg(ni + 1);
       if (inside && cnt > 0) {
         int st = __ldg(ni + 2);
+        L_ROLL
         for (int k = 0; k < cnt; ++k) visit(__ldg(S.items + st + k));
       }
       node = (inside && cnt == 0) ? node + 1 : __ldg(ni);
@@ -660,6 +675,7 @@ L_DEV int d_find(const DScene& S, int v, const NF* x) {
 }
 L_DEV int d_locate(const DScene& S, const NF* x) {
   int v = S.n;
+  L_ROLL
   for (int guard = 0; guard < 64; ++guard) {
     int f = d_find(S, v, x);
     if (f < 0) return v;
@@ -667,21 +683,24 @@ L_DEV int d_locate(const DScene& S, const NF* x) {
   }
   return v;
 }
+template <int TORUS>
 L_DEV int d_find_ray(const DScene& S, int v, const NF* od, const NF* dd, NF t, int excl, NF pad) {
   NF x[3] = {od[0] + t * dd[0], od[1] + t * dd[1], od[2] + t * dd[2]};
   int g = -1;
   d_point_scan(S, v, x, pad, [&](int i) {
-    if (d_level_wins(S, i, g, excl) && d_ray_holds(S, i, od, dd, t)) g = i;
+    if (d_level_wins(S, i, g, excl) && d_ray_holds<TORUS>(S, i, od, dd, t)) g = i;
   });
   return g;
 }
+template <int TORUS>
 L_DEV int d_settle(const DScene& S, int v, const NF* od, const NF* dd, NF t, int crossed, NF pad, int* moved) {
   int v_ = v, held = 0;
+  L_ROLL
   for (int guard = 0; guard < 256; ++guard) {
     int vi = v_ < S.n - 1 ? v_ : S.n - 1;
     int test = !held && v_ < S.n && v_ != crossed;
-    int ins = !test || d_ray_holds(S, vi, od, dd, t);
-    int f = ins ? d_find_ray(S, v_, od, dd, t, crossed, pad) : -1;
+    int ins = !test || d_ray_holds<TORUS>(S, vi, od, dd, t);
+    int f = ins ? d_find_ray<TORUS>(S, v_, od, dd, t, crossed, pad) : -1;
     int nv = ins ? (f >= 0 ? f : v_) : d_parent(S, v_ < S.n ? v_ : S.n);
     held = ins && f >= 0;
     if (f < 0 && ins) break;
@@ -701,6 +720,7 @@ L_DEV int d_find_x(const DScene& S, int v, const NF* x) {
 }
 L_DEV int d_locate_x(const DScene& S, const NF* x) {
   int v = S.n;
+  L_ROLL
   for (int guard = 0; guard < 64; ++guard) {
     int f = d_find_x(S, v, x);
     if (f < 0) return v;
@@ -712,16 +732,17 @@ L_DEV int d_find_ray_x(const DScene& S, int v, const NF* od, const NF* dd, NF t,
   NF x[3] = {od[0] + t * dd[0], od[1] + t * dd[1], od[2] + t * dd[2]};
   int g = -1;
   d_point_scan_x(S, v, x, pad, [&](int i) {
-    if (d_level_wins(S, i, g, excl) && !d_is_anc(S, i, v) && d_ray_holds(S, i, od, dd, t)) g = i;
+    if (d_level_wins(S, i, g, excl) && !d_is_anc(S, i, v) && d_ray_holds<1>(S, i, od, dd, t)) g = i;
   });
   return g;
 }
 L_DEV int d_settle_x(const DScene& S, int v, const NF* od, const NF* dd, NF t, int crossed, NF pad, int* moved) {
   int v_ = v, held = 0;
+  L_ROLL
   for (int guard = 0; guard < 256; ++guard) {
     int vi = v_ < S.n - 1 ? v_ : S.n - 1;
     int test = !held && v_ < S.n && v_ != crossed;
-    int ins = !test || d_ray_holds(S, vi, od, dd, t);
+    int ins = !test || d_ray_holds<1>(S, vi, od, dd, t);
     int f = ins ? d_find_ray_x(S, v_, od, dd, t, crossed, pad) : -1;
     int nv = ins ? (f >= 0 ? f : v_) : d_parent(S, v_ < S.n ? v_ : S.n);
     held = ins && f >= 0;
@@ -911,6 +932,7 @@ L_DEV Best d_mesh_visit(const DScene& S, const Ctx& c, int ch0, int i, Best b) {
   }
   const Shear h = d_shear(c.dd);
   const NF tol = N_FACET_BEHIND_BANDS * c.band;
+  L_ROLL
   for (int q = 0; q < kn; ++q) {
     NF t_k, nd, s0;
     int ok = d_crossing(S, c, h, k0 + q, &t_k, &nd, &s0);
@@ -984,6 +1006,7 @@ L_DEV Best d_enter_x(const DScene& S, const Ctx& c, int has_own, int vi) {
   int lp = 0, lend = 0;  // the current leaf's items still to visit: S.items[lp, lend)
   int started = 0;
   int pending = has_own;
+  L_ROLL
   for (;;) {
     int item = -1, is_own = 0;
     if (pending) {
@@ -1000,6 +1023,7 @@ L_DEV Best d_enter_x(const DScene& S, const Ctx& c, int has_own, int vi) {
           node = (tin <= tout && tout >= c.t_lo && tin <= d_min(b.t, c.t_bound) + c.band) ? n0 : -1;
         }
       }
+      L_ROLL
       while (item < 0) {
         if (lp < lend) {
           item = __ldg(S.items + lp++);
@@ -1007,6 +1031,7 @@ L_DEV Best d_enter_x(const DScene& S, const Ctx& c, int has_own, int vi) {
         }
         if (node < 0) {
           NF lim = d_min(b.t, c.t_bound) + c.band;
+          L_ROLL
           while (sp > 0 && tins[sp - 1] > lim) sp--;
           if (sp == 0) break;
           sp--;
@@ -1110,6 +1135,7 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
 #endif
   int started = 0;     // the root has been tested
   int pending = has_own;
+  L_ROLL
   for (;;) {
     int item = -1, is_own = 0;
     if (pending) {
@@ -1130,6 +1156,7 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
 #endif
         }
       }
+      L_ROLL
       while (item < 0) {
 #if NAV_IS64
         if (lp < lend) {
@@ -1145,6 +1172,7 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
 #endif
         if (node == -1) {
           NF lim = d_min(b.t, c.t_bound) + c.band;
+          L_ROLL
           while (sp > 0 && tins[sp - 1] > lim) sp--;
           if (sp == 0) break;
           sp--;
@@ -1227,6 +1255,7 @@ L_DEV Query d_query(const DScene& S, const NF* o, const NF* d, int vol, NF t_max
   NF pz_tp0 = N_HUGE, pz_tp1 = N_HUGE, pz_tin = 0.0f;
   int pz_np = 0, pz_vend = vol, pz_hit = 0, pz_vat = vol, pz_zc = 0, pz_vin = vol;
   int guard = 0;
+  L_ROLL
   while (!done) {
     NF band = d_band(xa + n_abs(t_lo));
     int vi = v < OUT - 1 ? v : OUT - 1;
@@ -1285,7 +1314,7 @@ L_DEV Query d_query(const DScene& S, const NF* o, const NF* d, int vol, NF t_max
       if (is_ch) { nxt = OUT + 1 + __ldg(S.mesh + MESH_HDR + 4 * (u_in - ch0) + 2); moved = 0; }
       else if (hit) {
         if constexpr ((TORUS & 1)) nxt = d_settle_x(S, nx0, od2, d, tr, unit_x, step + step, &moved);
-        else nxt = d_settle(S, nx0, od2, d, tr, unit_x, step + step, &moved);
+        else nxt = d_settle<TORUS>(S, nx0, od2, d, tr, unit_x, step + step, &moved);
       }
       else { nxt = nx0; moved = 0; }
     }
@@ -1420,6 +1449,7 @@ L_DEV NF d_reach_bound(const DScene& S, const NF* x, const float* d, int vol, in
     tout = d_min(tout, d_max(ta, tb));
   }
   if (!(tin <= 0.0f && s < tout && s < t_max)) return t_max;
+  L_ROLL
   for (int node = 0, guard = 0; node < S.n_fnode && guard < S.n_fnode; ++guard) {  // any sensor box on [0, T]
     NF ti, to;
     d_slab(S.fnode_f, node, x, inv, &ti, &to);

@@ -26,6 +26,7 @@ L_CALL float d_tab_k(const float* __restrict__ xe, int k, float E) {
   if (E <= __ldg(xe)) return __ldg(fv);
   if (E >= __ldg(xe + k - 1)) return __ldg(fv + k - 1);
   int i = 1;
+  L_ROLL
   while (i < k - 1 && __ldg(xe + i) <= E) ++i;
   float x0 = __ldg(xe + i - 1), x1 = __ldg(xe + i);
   float f0 = __ldg(fv + i - 1), f1 = __ldg(fv + i);
@@ -62,6 +63,7 @@ L_DEV float d_group_index(const DScene& S, const float* __restrict__ pool, int t
   if (kk == 1) return __ldg(n);
   int k = kk - 1;
   int p = 0;
+  L_ROLL
   while (p < k + 1 && d_eg(e, k, p) <= E) ++p;
   p = p < 1 ? 1 : (p > k ? k : p);
   float x0 = d_eg(e, k, p - 1), x1 = d_eg(e, k, p);
@@ -288,6 +290,7 @@ L_DEV void d_type_eval(const DScene& S, const float* __restrict__ pool, int row,
   ev.sigma = 0.1f;
   ev.amps[0] = cf(-1.0f, 0.0f); ev.amps[1] = cf(1.0f, 0.0f); ev.amps[2] = cf(1.0f, 0.0f); ev.amps[3] = cf(1.0f, 0.0f);
   if (G > 0)
+    L_ROLL
     for (int p = 0; p < P; ++p) {
 #pragma unroll
       for (int o = 0; o < N_OUT; ++o) dprobs[p][o] = 0.0f;
@@ -359,6 +362,7 @@ L_DEV void d_type_eval(const DScene& S, const float* __restrict__ pool, int row,
   ev.detect = a * col[LUMEN_COL_EFF];
   ev.sigma = __ldg(ri + LUMEN_RI_GLISUR) ? 1.0f - col[LUMEN_COL_POLISH] : col[LUMEN_COL_SIGMA];
   if (G > 0) {
+    L_ROLL
     for (int p = 0; p < P; ++p) {
       float dc[LUMEN_N_COL];
 #pragma unroll
@@ -444,6 +448,7 @@ L_DEV void d_unified_facet(float sigma, const float* V, Key key, float* m, int* 
   float fmax = d_min(1.0f, 4.0f * sigma);
   float a = 0.0f, u2 = 0.5f;
   int ok = 0;
+  L_ROLL
   for (uint32_t t = 0; t < D_FACET_REDRAWS && !ok; ++t) {
     Key kt = fold_in(key, t);
     float u0 = uniform(kt, 0), u1 = uniform(kt, 1);
@@ -589,6 +594,7 @@ L_DEV void d_facet_path(float sigma, const float* wi, const float* n, float r0, 
   float V[3];
   d_to_local(mwi, n, V);
   float w[3] = {wi[0], wi[1], wi[2]};
+  L_ROLL
   for (uint32_t k = 0; k < D_FACET_PATH; ++k) {
     float m[3];
     d_unified_facet(sigma, V, fold_in(key, k), m, capped);
@@ -638,6 +644,7 @@ L_DEV void d_glisur_facet(float r, const float* V, Key key, float e, float* m, i
   int shell = e > 0.0f && uniform(fold_in(key, D_SHELL_STREAM), 0) < e;
   float M[3] = {0.0f, 0.0f, 1.0f};
   int ok = 0;
+  L_ROLL
   for (uint32_t t = 0; t < D_FACET_REDRAWS && !ok; ++t) {
     Key kt = fold_in(key, t);
     float u0 = uniform(kt, 0), u1 = uniform(kt, 1), u2 = uniform(kt, 2);
@@ -721,6 +728,7 @@ L_DEV float d_glisur_metal_path(float r_ref, float r_live, const float* wi, cons
   d_to_local(mwi, n, V);
   float w[3] = {wi[0], wi[1], wi[2]};
   float lp = 0.0f, lr = 0.0f, dl = 0.0f;
+  L_ROLL
   for (uint32_t k = 0; k < D_FACET_PATH; ++k) {
     float m[3];
     d_glisur_facet(r_ref, V, fold_in(key, k), e, m, capped);
@@ -822,6 +830,7 @@ L_DEV float d_glisur_dielectric_path(float r_ref, float r_live, float n1, float 
   float er_r[3] = {er[0], er[1], er[2]}, ei_r[3] = {ei[0], ei[1], ei[2]};
   float lp = 0.0f, lr = 0.0f, dl = 0.0f;
   int far = 0;
+  L_ROLL
   for (uint32_t k = 0; k < D_FACET_PATH; ++k) {
     float N[3] = {side * n[0], side * n[1], side * n[2]};
     float na = side > 0.0f ? n1 : n2, nb = side > 0.0f ? n2 : n1;

@@ -69,6 +69,7 @@ L_DEV void d_diffuse(const DScene& S, int mi, const float* xs, const float* d0, 
   Key jkey = fold_in(vkey, D_JUMP_STREAM);
   const float zero[3] = {0.0f, 0.0f, 0.0f};
   int out = 0;
+  L_ROLL
   for (int j = 0; j < budget && !out; ++j) {
     Key kj = fold_in(jkey, (uint32_t)j);
     float u0 = uniform(kj, 0);
@@ -277,6 +278,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
     const int32_t* m = S.med_i + (size_t)mi * LUMEN_MED_I;
     int ta = __ldg(m + LUMEN_MI_ABS);
     float E = D_HC / ph.lam;
+    L_ROLL
     for (int p = 0; p < P; ++p) {
       dmu_abs[p] = 0.0f;
       if (ta >= 0 && ta == R.gt[p]) dmu_abs[p] = d_tab(S, R.live, ta, E) >= D_FLT_TINY ? -(ml.mu_abs * ml.mu_abs) : 0.0f;
@@ -312,6 +314,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
     int te = __ldg(S.row_i + (size_t)row * LUMEN_ROW_I + LUMEN_RI_COL + LUMEN_COL_EFF);
     need_eval = d_tab(S, R.live, te, D_HC / ph.lam) != 0.0f;
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < P; ++p) need_eval = need_eval || te == R.gt[p];
   }
   float dprobs[G > 0 ? G : 1][N_OUT], ddet[G > 0 ? G : 1];
@@ -332,6 +335,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
     le.sigma = 0.1f;
     re = le;
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < P; ++p) {
 #pragma unroll
         for (int o = 0; o < N_OUT; ++o) dprobs[p][o] = 0.0f;
@@ -344,6 +348,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
     le.detect = 0.0f;
     re.detect = 0.0f;
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < P; ++p) {
 #pragma unroll
         for (int o = 0; o < N_OUT; ++o) dprobs[p][o] = 0.0f;
@@ -386,6 +391,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
   dep.q = at_if ? ph.w * reach_live * att_if * p_det : 0.0f;
   float d_reach[G > 0 ? G : 1], d_att[G > 0 ? G : 1];
   if (G > 0)
+    L_ROLL
     for (int p = 0; p < P; ++p) {
       d_reach[p] = -(dmu_c[p] * dist) * reach_live;
       d_att[p] = -(dmu_abs[p] * dist) * att_if;
@@ -478,6 +484,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
       nx_w = nx_w * wj;
     }
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < P; ++p) {
         float dwp = (dch[p][cs] * e_l + mu_c_l * (-(dmu_c[p] * s) * e_l)) / path_r;
         if (!(path_r != 0.0f)) dwp = 0.0f;
@@ -576,6 +583,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
     if (G > 0) {
       int t_sig = row >= 0 ? __ldg(S.row_i + (size_t)row * LUMEN_ROW_I + LUMEN_RI_COL +
                                   (lobe_sign > 0.0f ? LUMEN_COL_SIGMA : LUMEN_COL_POLISH)) : -1;
+      L_ROLL
       for (int p = 0; p < P; ++p) {
         float dpl = dprobs[p][os_];
         float dr_live = drawn ? (pp != 0.0f ? dpl / pp : 0.0f) : 0.0f;
@@ -676,6 +684,7 @@ L_DEV void d_post(const Run& R, PhotonT<NF>& ph, float* dw, const PreT<NF>& pr, 
   ph.w = alive ? w_new : 0.0f;
   ph.wr = alive ? wr_new : 0.0f;
   if (G > 0)
+    L_ROLL
     for (int p = 0; p < P; ++p) {
       float v = kept ? nx_dw[p] / p_kept : (lostr ? 0.0f : nx_dw[p]);
       dw[p] = alive ? v : 0.0f;
@@ -719,6 +728,7 @@ L_DEV void d_born(const Run& R, PhotonT<NF>& ph, float* dw, int bp, Dep& dep, fl
   dep.q = ph.w * d;
   dep.time = ph.t;
   if (G > 0)
+    L_ROLL
     for (int p = 0; p < P; ++p) dq[p] = dw[p] * d + ph.w * ddet[p];
 #pragma unroll
   for (int k = 0; k < 8; ++k) dep.fates[k] = 0.0f;
@@ -749,6 +759,7 @@ L_DEV void d_born(const Run& R, PhotonT<NF>& ph, float* dw, int bp, Dep& dep, fl
   ph.w = 0.0f;
   ph.wr = 0.0f;
   if (G > 0)
+    L_ROLL
     for (int p = 0; p < P; ++p) dw[p] = 0.0f;
   ph.vertex += 1;
 }
@@ -781,6 +792,7 @@ L_DEV float d_gaussian(float u) {
 
 L_DEV int d_event_of(const int64_t* first, int n_ev, int64_t gid) {
   int lo = 0, hi = n_ev - 1;
+  L_ROLL
   while (lo < hi) {
     int mid = (lo + hi + 1) / 2;
     if (__ldg((const long long*)first + mid) <= gid) lo = mid; else hi = mid - 1;
@@ -818,23 +830,29 @@ L_DEV void d_scint_row(const DScene& S, const float* __restrict__ live, const fl
   d_scint_shares(S, live, m, fl);
   d_scint_shares(S, ref, m, q);
   int n_off = 0;
+  L_ROLL
   for (int i = 0; i < nc; ++i) n_off += q[i] <= 0.0f;
   if (n_off > 0) {  // the defensive mixture: a component of share 0 gets e / (1 - e) / n, then all normalised
     float eps = (float)(0.01 / 0.99) / (float)n_off, sum = 0.0f;
+    L_ROLL
     for (int i = 0; i < nc; ++i) { q[i] = q[i] <= 0.0f ? eps : q[i]; sum = i == 0 ? q[i] : sum + q[i]; }
+    L_ROLL
     for (int i = 0; i < nc; ++i) q[i] = q[i] / sum;
   }
   const float u_lam = uniform(rk, 0), u_d0 = uniform(rk, 1), u_d1 = uniform(rk, 2), u_c = uniform(rk, 3);
   const float u_t = uniform(rk, 4);
   int c = 0;
   float cs = 0.0f;
+  L_ROLL
   for (int i = 0; i + 1 < nc; ++i) {
     cs = i == 0 ? q[0] : cs + q[i];
     c += u_c >= cs;
   }
   int nxt = nc, last = 0;  // lit: the first share above zero at or after c, else the last one
+  L_ROLL
   for (int i = nc - 1; i >= 0; --i)
     if (q[i] > 0.0f && i >= c) nxt = i;
+  L_ROLL
   for (int i = 0; i < nc; ++i)
     if (q[i] > 0.0f) last = i;
   c = nxt < last ? nxt : last;

@@ -225,10 +225,12 @@ __device__ __forceinline__ int deposit(const Tally& T, int e, const Dep& dep, co
   }
   if (G > 0) {
     if (T.jac)
+      L_ROLL
       for (int p = 0; p < T.P; ++p) atomicAdd(T.jac + ix * T.P + p, (double)dq[p] * w0);
     if (T.cot) {
       double c = T.cot[ix];
       if (c != 0.0)
+        L_ROLL
         for (int p = 0; p < T.P; ++p) atomicAdd(T.grads + p, c * (double)dq[p] * w0);
     }
   }
@@ -348,6 +350,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
       w0 = ex.w0;
       pt = ex.pt;
       if (G > 0)
+        L_ROLL
         for (int p = 0; p < L.R.P; ++p) dw[p] = L.wv_dw[(size_t)p * L.wv_W + i];
       active = 1;
     }
@@ -376,6 +379,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
           pt.n = 0;
           pt.pid = (unsigned)g;
           if (G > 0)
+            L_ROLL
             for (int p = 0; p < L.R.P; ++p) dw[p] = 0.0f;
           if (ANALOG) {  // run.py:319: one uniform of its own stream, open with probability k (state.py:58)
             float u = uniform(fold_in(pkey, D_ANALOG_STREAM), 0);
@@ -511,6 +515,7 @@ __global__ void __launch_bounds__(256) k_wave_fill(Launch L, Wave V) {
   wave_new<EXT>(L, i, ph, ex);
   wv_st(V.ph, V.W, i, ph);
   wv_st(V.ex, V.W, i, ex);
+  L_ROLL
   for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = 0.0f;
   V.out[i] = i;
 }
@@ -594,6 +599,7 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
     wv_ld(V.ph, V.W, i, ph);
     wv_ld(V.ex, V.W, i, ex);
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < L.R.P; ++p) dw[p] = V.dw[(size_t)p * V.W + i];
     Ana an;
     const int bp = BORN ? d_born_entry(L.R.S, ph) : -2;
@@ -642,6 +648,7 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
       if (g < (unsigned long long)L.n) {
         wave_new<EXT>(L, (int64_t)g, ph, ex);
         if (G > 0)
+          L_ROLL
           for (int p = 0; p < L.R.P; ++p) dw[p] = 0.0f;
         act = 1;
       }
@@ -651,6 +658,7 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
     wv_st(V.ph, V.W, i, ph);
     wv_st(V.ex, V.W, i, ex);
     if (G > 0)
+      L_ROLL
       for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = dw[p];
   }
   // the next round's list: the block's slots that go on, in the order they came in, one atomic a block
