@@ -563,6 +563,38 @@ L_DEV NF d_face_dist(const DScene& S, int item, int leaf, int face, const NF* x)
   return d_leaf_dist(S, vI(S, i, LUMEN_VI_KIND), leaf, face, xl);
 }
 
+// d_hit_grad and d_face_dist at one point, what they share computed once (the settle's share and the query's last part
+// were 38 % of the tank's query, chains of loads; d_query keeps the gradient and normal taken here for its result)
+L_DEV void d_hit_grad_dist(const DScene& S, int item, int leaf, int face, const NF* x, NF* gw, NF* dist) {
+  const int i = d_clampv(S, item), kind = vI(S, i, LUMEN_VI_KIND);
+  NF xl[3], g[3], f;
+  d_to_local_pt(S, i, x, xl);
+  const int gi = __ldg(S.kind_i + (size_t)kind * LUMEN_KIND_I) + (leaf > 0 ? leaf : 0);
+  const NF* lf = NAV_LEAF(S) + (size_t)gi * LUMEN_LEAF_F;
+  const int32_t* li = S.leaf_i + (size_t)gi * LUMEN_LEAF_I;
+  if (face >= 1) {
+    const NF* p = NAV_PLANE(S) + (size_t)(__ldg(li + 1) + face - 1) * LUMEN_PLANE_F;
+    g[0] = __ldg(p); g[1] = __ldg(p + 1); g[2] = __ldg(p + 2);
+    NF q[3] = {xl[0] - __ldg(lf + 0), xl[1] - __ldg(lf + 1), xl[2] - __ldg(lf + 2)};
+    f = g[0] * q[0] + g[1] * q[1] + g[2] * q[2] - __ldg(p + 3);
+    *dist = n_abs(f) / d_safe_norm(g);
+  } else if (__ldg(li) == 2) {
+    d_leaf_grad(S, kind, leaf, face, xl, g);
+    *dist = d_leaf_dist(S, kind, leaf, face, xl);
+  } else {
+    NF y[3] = {xl[0] - __ldg(lf + 3), xl[1] - __ldg(lf + 4), xl[2] - __ldg(lf + 5)}, Ay[3];
+    d_Av(lf + LUMEN_LF_A, y, Ay);
+    const NF* b = lf + LUMEN_LF_B;
+    const NF b0 = __ldg(b), b1 = __ldg(b + 1), b2 = __ldg(b + 2);
+    f = (d_dot(y, Ay) + 2.0f * (b0 * y[0] + b1 * y[1] + b2 * y[2])) + __ldg(lf + LUMEN_LF_C);
+    g[0] = 2.0f * (Ay[0] + b0);
+    g[1] = 2.0f * (Ay[1] + b1);
+    g[2] = 2.0f * (Ay[2] + b2);
+    *dist = n_abs(f) / d_safe_norm(g);
+  }
+  d_to_world_dir(S, i, g, gw);
+}
+
 L_DEV int d_srf_pack(const DScene& S, int item, int leaf, int face, int o, int e) {
   if (item < 0 || leaf < 0 || face < 0) return item;
   return S.SU + ((item * S.LM + leaf) * S.FM + face) * 4 + 2 * o + e;
@@ -1107,10 +1139,10 @@ L_DEV void d_slab_box(const float* bx, const NF* o, const NF* inv, NF* tin, NF* 
 
 // The candidate entries of volume c.v along the ray (navigate.py:482 enter, :465 _group, :430 _node): the volume's own
 // solid first (has_own), then its BVH depth first, the nearer child first and the farther onto the stack with its
-// entry t, the stack's entries past the best event so far dropped, each leaf's items in turn (a leaf holds one or
-// more). The float32 navigator walks the node records (S.node_w: per inner node both children's boxes and codes in
-// 64 B, four 16-byte loads a level); the float64 one the node arrays (a child's box and its right sibling's index
-// read from the node).
+// entry t, what lies past the best event so far dropped, each leaf's items in turn (a leaf holds one or more). One call
+// site of the visit.
+#if NAV_IS64
+// The float64 navigator walks the node arrays (a child's box and its right sibling's index read from the node).
 template <int TORUS>
 L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
   if constexpr (TORUS == 3) return d_enter_x(S, c, has_own, vi);
@@ -1126,13 +1158,8 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
   int stack[D_STACK];
   NF tins[D_STACK];
   int sp = 0;
-#if NAV_IS64
   int node = -1;       // the traversal's next node (-1: pop or done)
   int lp = 0, lend = 0;  // the current leaf's items still to visit: S.items[lp, lend)
-#else
-  int node = -1;       // the next node's code: an inner node's index, -2 - p a leaf's item list at S.witem + p, -1 none
-  int lp = -1;         // the current leaf's next item in S.witem (-1: none)
-#endif
   int started = 0;     // the root has been tested
   int pending = has_own;
   L_ROLL
@@ -1149,27 +1176,15 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
           NF tin, tout;
           d_slab(NAV_NODE(S), n0, c.od, inv, &tin, &tout);
           const int meets = tin <= tout && tout >= c.t_lo && tin <= d_min(b.t, c.t_bound) + c.band;
-#if NAV_IS64
           node = meets ? n0 : -1;
-#else
-          node = meets ? __float_as_int(__ldg(S.node_w + (size_t)n0 * 4 + 3).z) : -1;  // the root's own code
-#endif
         }
       }
       L_ROLL
       while (item < 0) {
-#if NAV_IS64
         if (lp < lend) {
           item = __ldg(S.items + lp++);
           break;
         }
-#else
-        if (lp >= 0) {
-          item = __ldg(S.witem + lp);
-          lp = __ldg(S.witem + lp + 1) >= 0 ? lp + 1 : -1;
-          break;
-        }
-#endif
         if (node == -1) {
           NF lim = d_min(b.t, c.t_bound) + c.band;
           L_ROLL
@@ -1178,7 +1193,6 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
           sp--;
           node = stack[sp];
         }
-#if NAV_IS64
         const int32_t* ni = S.node_i + (size_t)node * LUMEN_NODE_I;
         int cnt = __ldg(ni + 1);
         if (cnt > 0) {  // a leaf: its items in turn
@@ -1192,20 +1206,6 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
         NF tl, tlo, tr, tro;
         d_slab(NAV_NODE(S), lc, c.od, inv, &tl, &tlo);
         d_slab(NAV_NODE(S), rc, c.od, inv, &tr, &tro);
-#else
-        if (node <= -2) {  // a leaf: its items in turn
-          lp = -2 - node;
-          node = -1;
-          continue;
-        }
-        const float4* nw = S.node_w + (size_t)node * 4;
-        const float4 w0 = __ldg(nw), w1 = __ldg(nw + 1), w2 = __ldg(nw + 2), w3 = __ldg(nw + 3);
-        const float bl[6] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y}, br[6] = {w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
-        const int lc = __float_as_int(w3.x), rc = __float_as_int(w3.y);
-        NF tl, tlo, tr, tro;
-        d_slab_box(bl, c.od, inv, &tl, &tlo);
-        d_slab_box(br, c.od, inv, &tr, &tro);
-#endif
         NF lim = d_min(b.t, c.t_bound) + c.band;
         int hl = tl <= tlo && tlo >= c.t_lo && tl <= lim;
         int hr = tr <= tro && tro >= c.t_lo && tr <= lim;
@@ -1226,6 +1226,126 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
   }
   return b;
 }
+#else
+// The float32 navigator walks the node records (S.node_w: per inner node both children's boxes and codes in 64 B, four
+// 16-byte loads a level), apart from the visits: the leaves a ray meets are set aside, up to D_CAND of them, and visited
+// once the walk has ended or the list is full, those past an event found since left out. A warp's lanes meet their leaves
+// after different numbers of nodes; visited as they were met, the warp waited for its slowest lane's next leaf before
+// each visit. The votes hold the lanes that entered together to one node, and to one visit, at a time: without
+// them the compiler's branches let the lanes run apart (7 of 32 lanes an instruction on the tank, 16 in the loop that
+// visited as it walked, 20 here; its 2^24 photons 55.6, 40.1 and 39.0 ms). Lists of 4 measured the same, visits at the
+// first leaf (with votes) 42.0 ms.
+#define D_CAND 6
+template <int TORUS>
+L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
+  if constexpr (TORUS == 3) return d_enter_x(S, c, has_own, vi);
+  const unsigned mask = __activemask();
+  Best b = {N_HUGE, -1, -1, -1, 0, 0};
+  const int ch0 = (TORUS & 1) ? m_ch0(S) : 0x7fffffff;  // the extended instantiation: mesh chunks among the items
+  NF inv[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    NF dv = c.dd[a];
+    inv[a] = 1.0f / (n_abs(dv) < N_TINY_DIR ? (dv < 0.0f ? -N_TINY_DIR : N_TINY_DIR) : dv);
+  }
+  int stack[D_STACK], cand[D_CAND];
+  NF tins[D_STACK], ctin[D_CAND];
+  int sp = 0, nc = 0, ci = 0;  // the stack's nodes; the leaves set aside and those of them taken
+  int node = -1;               // the next inner node, -1: pop
+  int lp = -1;                 // the current leaf's next item in S.witem (-1: none)
+  int started = 0;             // the root has been tested
+  int item = has_own ? vi : -1, is_own = has_own;
+  for (;;) {
+    L_ROLL
+    while (__any_sync(mask, item >= 0)) {  // the items set aside
+      if (item >= 0) {
+        if ((TORUS & 1) && item >= ch0 && !is_own) b = d_mesh_visit(S, c, ch0, item, b);
+        else b = d_unit_visit<TORUS>(S, c, item, b, is_own);
+        is_own = 0;
+        item = -1;
+        if (lp < 0) {
+          const NF lim = d_min(b.t, c.t_bound) + c.band;
+          L_ROLL
+          while (ci < nc && ctin[ci] > lim) ++ci;
+          if (ci < nc) lp = cand[ci++];
+        }
+        if (lp >= 0) {
+          item = __ldg(S.witem + lp);
+          lp = __ldg(S.witem + lp + 1) >= 0 ? lp + 1 : -1;
+        }
+      }
+    }
+    const NF lim = d_min(b.t, c.t_bound) + c.band;
+    nc = ci = 0;
+    int walking = 1;
+    if (!started) {
+      started = 1;
+      const int n0 = vI(S, c.v, LUMEN_VI_NODE0), n1 = vI(S, c.v, LUMEN_VI_NODE1);
+      if (n0 < n1) {
+        NF tin, tout;
+        d_slab(NAV_NODE(S), n0, c.od, inv, &tin, &tout);
+        if (tin <= tout && tout >= c.t_lo && tin <= lim) {
+          node = __float_as_int(__ldg(S.node_w + (size_t)n0 * 4 + 3).z);  // the root's own code
+          if (node <= -2) {
+            cand[0] = -2 - node;
+            ctin[0] = tin;
+            nc = 1;
+            node = -1;
+          }
+        }
+      }
+    }
+    L_ROLL
+    while (__any_sync(mask, walking)) {
+      if (walking && node < 0) {
+        L_ROLL
+        while (sp > 0 && tins[sp - 1] > lim) sp--;
+        if (sp > 0) node = stack[--sp];
+        else walking = 0;
+      }
+      if (walking) {
+        const float4* nw = S.node_w + (size_t)node * 4;
+        const float4 w0 = __ldg(nw), w1 = __ldg(nw + 1), w2 = __ldg(nw + 2), w3 = __ldg(nw + 3);
+        const float bl[6] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y}, br[6] = {w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
+        const int lc = __float_as_int(w3.x), rc = __float_as_int(w3.y);
+        NF tl, tlo, tr, tro;
+        d_slab_box(bl, c.od, inv, &tl, &tlo);
+        d_slab_box(br, c.od, inv, &tr, &tro);
+        int hl = tl <= tlo && tlo >= c.t_lo && tl <= lim;
+        int hr = tr <= tro && tro >= c.t_lo && tr <= lim;
+        if (hl && lc < 0) {
+          cand[nc] = -2 - lc;
+          ctin[nc] = tl;
+          nc++;
+          hl = 0;
+        }
+        if (hr && rc < 0) {
+          cand[nc] = -2 - rc;
+          ctin[nc] = tr;
+          nc++;
+          hr = 0;
+        }
+        const int first = hl && (!hr || tl <= tr);
+        if (hl && hr && sp < D_STACK) {
+          stack[sp] = first ? rc : lc;
+          tins[sp] = first ? tr : tl;
+          sp++;
+        }
+        node = first ? lc : (hr ? rc : -1);
+        walking = nc <= D_CAND - 2;
+      }
+    }
+    if (nc > 0) {
+      lp = cand[0];
+      ci = 1;
+      item = __ldg(S.witem + lp);
+      lp = __ldg(S.witem + lp + 1) >= 0 ? lp + 1 : -1;
+    }
+    if (!__any_sync(mask, item >= 0)) break;
+  }
+  return b;
+}
+#endif
 
 // ------------------------------------------------------------------------------------------------ the query
 using Query = QueryT<NF>;
