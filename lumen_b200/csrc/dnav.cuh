@@ -1373,6 +1373,7 @@ L_DEV Query d_query(const DScene& S, const NF* o, const NF* d, int vol, NF t_max
   int rec_item = -1, rec_leaf = -1, rec_face = -1, rec_zero = 0, rec_vb = vol, rec_vis = 0;
   int cur = cls0;
   NF pz_tp0 = N_HUGE, pz_tp1 = N_HUGE, pz_tin = 0.0f;
+  NF rec_g[3] = {0.0f, 0.0f, 0.0f}, rec_n[3] = {0.0f, 0.0f, 0.0f};  // the last hit's gradient and normal (a leaf's)
   int pz_np = 0, pz_vend = vol, pz_hit = 0, pz_vat = vol, pz_zc = 0, pz_vin = vol;
   int guard = 0;
   L_ROLL
@@ -1421,14 +1422,14 @@ L_DEV Query d_query(const DScene& S, const NF* o, const NF* d, int vol, NF t_max
         NF x[3] = {o[0] + t_c * d[0], o[1] + t_c * d[1], o[2] + t_c * d[2]};
         int itm = is_own ? vi : uc;
         int lf = l_in > 0 ? l_in : 0;
-        NF g[3];
-        d_hit_grad(S, itm, lf, f_in, x, g);
-        NF gn = d_safe_norm(g);
-        NF n_[3] = {g[0] / gn, g[1] / gn, g[2] / gn};
-        NF m = d_face_dist(S, itm, lf, f_in, x) + D_RELOCATE_BANDS * d_band(d_maxabs3(x));
-        NF sg = d_dot(n_, d) < 0.0f ? -1.0f : 1.0f;
+        NF fd;
+        d_hit_grad_dist(S, itm, lf, f_in, x, rec_g, &fd);
+        NF gn = d_safe_norm(rec_g);
+        rec_n[0] = rec_g[0] / gn; rec_n[1] = rec_g[1] / gn; rec_n[2] = rec_g[2] / gn;
+        NF m = fd + D_RELOCATE_BANDS * d_band(d_maxabs3(x));
+        NF sg = d_dot(rec_n, d) < 0.0f ? -1.0f : 1.0f;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) od2[a] = o[a] + m * sg * n_[a];
+        for (int a = 0; a < 3; ++a) od2[a] = o[a] + m * sg * rec_n[a];
       }
       NF tr = off ? t_c : t_c + step;
       if (is_ch) { nxt = OUT + 1 + __ldg(S.mesh + MESH_HDR + 4 * (u_in - ch0) + 2); moved = 0; }
@@ -1498,13 +1499,17 @@ L_DEV Query d_query(const DScene& S, const NF* o, const NF* d, int vol, NF t_max
       }
     }
   }
-  NF px = bt < N_HUGE ? bt : 0.0f;
-  NF xh[3] = {o[0] + px * d[0], o[1] + px * d[1], o[2] + px * d[2]};
-  NF g[3];
-  if constexpr ((TORUS & 1)) d_hit_grad_m(S, ch0, bi, bl > 0 ? bl : 0, bf, xh, g);
-  else d_hit_grad(S, bi, bl > 0 ? bl : 0, bf, xh, g);
-  NF gn = d_safe_norm(g);
-  NF nrm[3] = {g[0] / gn, g[1] / gn, g[2] / gn};
+  // the normal and the gradient at the hit: a leaf's were taken as the step left it (the same point); a mesh triangle's
+  // here; an event without a surface of its own (bl < 0) has neither, its surface code and normal read neither
+  NF g[3] = {rec_g[0], rec_g[1], rec_g[2]}, nrm[3] = {rec_n[0], rec_n[1], rec_n[2]};
+  if constexpr ((TORUS & 1)) {
+    if (bi >= ch0 && bl >= 0) {
+      const NF xh[3] = {0.0f, 0.0f, 0.0f};  // a triangle's normal is the same everywhere on it
+      d_hit_grad_m(S, ch0, bi, bl, bf, xh, g);
+      NF gn = d_safe_norm(g);
+      nrm[0] = g[0] / gn; nrm[1] = g[1] / gn; nrm[2] = g[2] / gn;
+    }
+  }
   NF fb[3] = {-d[0], -d[1], -d[2]};
   if (sn) {
     int sat = hit && zero && bl < 0 && kn0 && bt <= 0.0f;

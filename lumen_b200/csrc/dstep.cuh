@@ -173,8 +173,8 @@ L_DEV float d_ratio(float live, float ref) { return ref != 0.0f ? live / ref : 0
 // state after the fill is written back into the photon.
 template <class NF>
 struct PreT {
-  Key vkey;
   NF b0;  // the band at the start, in the navigator's precision (step.py:252)
+  Key vkey;
   float s;
   Med ml, mr;
 };
@@ -182,8 +182,9 @@ using Pre = PreT<float>;
 
 // the step up to its query: the stuck push, the vertex key, the polarisation fill, the media, the free path
 // (step.py:318 _step_context, :245 _recover)
+// Returns whether it changed the photon (the push or the fill).
 template <int EXT = 0, class NF>
-L_DEV void d_pre(const Run& R, PhotonT<NF>& ph, Key pkey, PreT<NF>& pr) {
+L_DEV int d_pre(const Run& R, PhotonT<NF>& ph, Key pkey, PreT<NF>& pr) {
   const DScene& S = R.S;
   pr.b0 = nav_band(nav_maxabs3(ph.x));
   int stuck = ph.alive && ph.nz >= D_ZSBP;
@@ -196,12 +197,14 @@ L_DEV void d_pre(const Run& R, PhotonT<NF>& ph, Key pkey, PreT<NF>& pr) {
     ph.srf = -1;
   }
   pr.vkey = fold_in(pkey, (uint32_t)ph.vertex);
-  if (d_dot(ph.er, ph.er) + d_dot(ph.ei, ph.ei) < D_ZERO_STATE)
+  const int fill = d_dot(ph.er, ph.er) + d_dot(ph.ei, ph.ei) < D_ZERO_STATE;
+  if (fill)
     d_fill(ph.d, ph.er, ph.ei, uniform(fold_in(pr.vkey, D_POL_STREAM), 0));
   int mi = __ldg(S.cls_medium + ph.cls);
   pr.ml = d_medium_at(S, R.live, ph.lam, mi);
   pr.mr = R.shared ? pr.ml : d_medium_at(S, R.ref, ph.lam, mi);
   pr.s = -l_log(uniform(pr.vkey, 0)) / d_max(pr.mr.mu_c, D_FLOOR32);
+  return stuck || fill;
 }
 
 // the step's query, bounded just past the free path where no sensor can be met (step.py:260 _query with

@@ -139,6 +139,7 @@ struct Launch {
   // wv_list[t], t < *wv_n; wv_W slots in the pool), or wv_W = 0
   const uint32_t* wv_ph;
   const uint32_t* wv_ex;
+  const uint32_t* wv_pt;
   const float* wv_dw;
   const int32_t* wv_list;
   const unsigned* wv_n;
@@ -270,18 +271,28 @@ __global__ void k_event_locate(DScene S, LumenSource src, int32_t* ev_vol) {
   ev_vol[e] = nav_locate<EXT>(S, x);
 }
 
-struct WaveExtra {  // what a slot carries besides the photon: its key, event, row weight and sensor-sum cache
+struct WaveExtra {  // what a slot carries besides the photon and its sensor sums: its key, event and row weight
   Key pkey;
-  int ev, pad;
-  double w0;
-  PhotonTally pt;
+  int ev;
+  float w0;
+};
+// what the step reads of the query (QueryT without what only the parity entry points read; the volume and class it
+// started in are the photon's)
+template <class NF>
+struct WaveQuery {
+  NF t;
+  int hit;  // bit 0 hit, bit 1 cont
+  int vol_after, vol_before, cls_before, cls_after;
+  float normal[3], t_pass0, t_pass1;
+  int vol_at, srf;
 };
 
 struct Wave {  // the records of the navigator's precision NF
   uint32_t* ph;     // W x sizeof(PhotonT<NF>) / 4
   uint32_t* ex;     // W x sizeof(WaveExtra) / 4
-  uint32_t* pre;    // W x sizeof(PreT<NF>) / 4
-  uint32_t* q;      // W x sizeof(QueryT<NF>) / 4
+  uint32_t* pt;     // W x sizeof(PhotonTally) / 4
+  uint32_t* pre;    // W x sizeof(PreT<NF>) / 4 (without mr where the live values are the reference)
+  uint32_t* q;      // W x sizeof(WaveQuery<NF>) / 4
   float* dw;        // W x LUMEN_MAX_GRAD (gradient runs)
   int W;
   // the round's live slots in[0, *n_in) and the next round's out[0, *n_out); mid: the same slots after the query, each
@@ -295,18 +306,21 @@ struct Wave {  // the records of the navigator's precision NF
   unsigned round;
 };
 
+// a record's words; `most`: its first words only
 template <class T>
-__device__ __forceinline__ void wv_ld(const uint32_t* b, int W, int i, T& v) {
+__device__ __forceinline__ void wv_ld(const uint32_t* b, int W, int i, T& v, size_t most = sizeof(T) / 4) {
   static_assert(sizeof(T) % 4 == 0, "word-major records hold whole words");
   uint32_t* w = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll
-  for (int k = 0; k < (int)(sizeof(T) / 4); ++k) w[k] = b[(size_t)k * W + i];
+  for (int k = 0; k < (int)(sizeof(T) / 4); ++k)
+    if (k < most) w[k] = b[(size_t)k * W + i];
 }
 template <class T>
-__device__ __forceinline__ void wv_st(uint32_t* b, int W, int i, const T& v) {
+__device__ __forceinline__ void wv_st(uint32_t* b, int W, int i, const T& v, size_t most = sizeof(T) / 4) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(&v);
 #pragma unroll
-  for (int k = 0; k < (int)(sizeof(T) / 4); ++k) b[(size_t)k * W + i] = w[k];
+  for (int k = 0; k < (int)(sizeof(T) / 4); ++k)
+    if (k < most) b[(size_t)k * W + i] = w[k];
 }
 
 // The persistent photon loop: a lane refill per step (src/lumen/run.py:81 SCHEDULE = "step").
@@ -345,10 +359,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
       WaveExtra ex;
       wv_ld(L.wv_ph, L.wv_W, i, ph);
       wv_ld(L.wv_ex, L.wv_W, i, ex);
+      wv_ld(L.wv_pt, L.wv_W, i, pt);
       pkey = ex.pkey;
       ev = ex.ev;
-      w0 = ex.w0;
-      pt = ex.pt;
+      w0 = (double)ex.w0;
       if (G > 0)
         L_ROLL
         for (int p = 0; p < L.R.P; ++p) dw[p] = L.wv_dw[(size_t)p * L.wv_W + i];
@@ -473,7 +487,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
 // round k_wave_query runs every live slot's step up to and including its navigator query, and k_wave_step the rest of
 // the step, the deposit, the photon's end and the slot's refill from the source. Each kernel is a part of the
 // megakernel's code with its own registers; the state crosses HBM between them, word-major (word k of slot i at
-// buf[k * W + i]) so that the loads and stores of neighbouring slots are contiguous.
+// buf[k * W + i]) so that the loads and stores of neighbouring slots are contiguous. A round moves what it must: the
+// query stores the photon only where its start changed it (131 words a step instead of 218), and of its result what the
+// step reads; the step's sensor sums are read where it deposits or ends. With the hit's gradient kept from the settle
+// (dnav.cuh), same box, ms: tank 2^24 photons 39.1 -> 35.1, 1,000,003 3.22 -> 2.86, ground wall with four tangents 10.3
+// -> 9.7, track events 12.8 -> 11.4, liquid-argon box 23.5 -> 21.8, float64 panel 3.93 -> 3.20, solids box 8.6 -> 8.2.
 //
 // The kernels run over lists of live slots, not over the pool: once the source is spent a photon's end leaves its lane
 // idle for every later round, and with one photon a slot that is from the second round on (measured before the lists:
@@ -493,11 +511,13 @@ __device__ __forceinline__ void wave_new(const Launch& L, int64_t g, PhotonT<NF>
   get_row(L, g, r);
   d_start<EXT>(L.R.S, r, ph);
   ex.pkey = fold_in(L.key, (uint32_t)(L.first_id + g));
-  ex.w0 = (double)r.w0;
+  ex.w0 = r.w0;
   ex.ev = r.event;
-  ex.pad = 0;
-  ex.pt.n = 0;
-  ex.pt.pid = (unsigned)g;
+}
+// a slot's sensor sums of a new photon: none yet
+__device__ __forceinline__ void wv_no_sums(uint32_t* b, int W, int i, unsigned pid) {
+  b[(size_t)(offsetof(PhotonTally, n) / 4) * W + i] = 0u;
+  b[(size_t)(offsetof(PhotonTally, pid) / 4) * W + i] = pid;
 }
 
 // every slot takes a photon: slot i the call's photon i (W at most the call's photons rounded up to a block)
@@ -515,6 +535,7 @@ __global__ void __launch_bounds__(256) k_wave_fill(Launch L, Wave V) {
   wave_new<EXT>(L, i, ph, ex);
   wv_st(V.ph, V.W, i, ph);
   wv_st(V.ex, V.W, i, ex);
+  wv_no_sums(V.pt, V.W, i, (unsigned)i);
   L_ROLL
   for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = 0.0f;
   V.out[i] = i;
@@ -544,11 +565,12 @@ __global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wav
     wv_ld(V.ph, V.W, i, ph);
     wv_ld(V.ex, V.W, i, pkey);  // the record's first words
     PreT<NF> pr;
-    d_pre<(TORUS & 1)>(L.R, ph, pkey, pr);
+    if (d_pre<(TORUS & 1)>(L.R, ph, pkey, pr)) wv_st(V.ph, V.W, i, ph);
     QueryT<NF> q = d_step_query<TORUS>(L.R, ph, pr);
-    wv_st(V.ph, V.W, i, ph);
-    wv_st(V.pre, V.W, i, pr);
-    wv_st(V.q, V.W, i, q);
+    WaveQuery<NF> wq = {q.t, q.hit | (q.cont << 1), q.vol_after, q.vol_before, q.cls_before, q.cls_after,
+                        {q.normal[0], q.normal[1], q.normal[2]}, q.t_pass0, q.t_pass1, q.vol_at, q.srf};
+    wv_st(V.pre, V.W, i, pr, L.R.shared ? offsetof(PreT<NF>, mr) / 4 : sizeof(pr) / 4);
+    wv_st(V.q, V.W, i, wq);
     bulk = pr.mr.mu_c > 0.0f && pr.s < q.t;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
@@ -591,6 +613,7 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
   unsigned c_ph = 0, c_steps = 0, c_dep = 0, c_trunc = 0, c_multi = 0, c_lost = 0;
   PhotonT<NF> ph;
   WaveExtra ex;
+  PhotonTally pt;
   float dw[G > 0 ? G : 1], dq[G > 0 ? G : 1];
   Dep dep;
   const int stepped = act;
@@ -607,31 +630,44 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
       d_born<G>(L.R, ph, dw, bp, dep, dq, an);
     } else {
       PreT<NF> pr;
+      WaveQuery<NF> wq;
+      wv_ld(V.pre, V.W, i, pr, L.R.shared ? offsetof(PreT<NF>, mr) / 4 : sizeof(pr) / 4);
+      wv_ld(V.q, V.W, i, wq);
+      if (L.R.shared) pr.mr = pr.ml;
       QueryT<NF> q;
-      wv_ld(V.pre, V.W, i, pr);
-      wv_ld(V.q, V.W, i, q);
+      q.t = wq.t;
+      q.hit = wq.hit & 1; q.cont = wq.hit >> 1;
+      q.vol_after = wq.vol_after; q.vol_before = wq.vol_before; q.vol_start = ph.vol;
+      q.cls_before = wq.cls_before; q.cls_after = wq.cls_after; q.cls_start = d_cls(L.R.S, ph.vol);
+      q.normal[0] = wq.normal[0]; q.normal[1] = wq.normal[1]; q.normal[2] = wq.normal[2];
+      q.t_pass0 = wq.t_pass0; q.t_pass1 = wq.t_pass1;
+      q.vol_at = wq.vol_at; q.srf = wq.srf;
       d_post<G>(L.R, ph, dw, pr, q, dep, dq, an);
     }
     c_steps++;
+    const double w0 = (double)ex.w0;
+    const int ends = !ph.alive || ph.vertex >= L.R.max_vertices;
+    if (dep.sensor >= 0 || ends) wv_ld(V.pt, V.W, i, pt);
     if (dep.sensor >= 0) {
-      const int m = deposit<G>(L.T, ex.ev, dep, dq, ex.w0, ex.pt);
+      const int m = deposit<G>(L.T, ex.ev, dep, dq, w0, pt);
       c_multi += m == 1;
       c_lost += m == 2;
       c_dep++;
+      if (!ends) wv_st(V.pt, V.W, i, pt);
     }
-    if (!ph.alive || ph.vertex >= L.R.max_vertices) {
-      flush_all(L.T, ex.ev, ex.pt);
-      if (L.R.rec && ph.last >= 0) d_record_head(L.R, ph.last, (float)ex.w0, ex.ev);
+    if (ends) {
+      flush_all(L.T, ex.ev, pt);
+      if (L.R.rec && ph.last >= 0) d_record_head(L.R, ph.last, ex.w0, ex.ev);
       if (ph.alive) {
-        trunc_w = (double)ph.w * ex.w0;
+        trunc_w = (double)ph.w * w0;
         c_trunc++;
       }
-      start_w = ex.w0;
+      start_w = w0;
       c_ph++;
       act = 0;
     }
   }
-  health_add(sh_health, dep, stepped ? ex.w0 : 0.0, stepped);
+  health_add(sh_health, dep, stepped ? (double)ex.w0 : 0.0, stepped);
   warp_add(sh_health + LUMEN_H_START, start_w);
   warp_add(sh_health + LUMEN_H_TRUNCATED, trunc_w);
   // the refill: free slots take consecutive photon ids, one atomic per warp
@@ -647,6 +683,8 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
       unsigned long long g = base + __popc(m & ((1u << lane) - 1u));
       if (g < (unsigned long long)L.n) {
         wave_new<EXT>(L, (int64_t)g, ph, ex);
+        wv_st(V.ex, V.W, i, ex);
+        wv_no_sums(V.pt, V.W, i, (unsigned)g);
         if (G > 0)
           L_ROLL
           for (int p = 0; p < L.R.P; ++p) dw[p] = 0.0f;
@@ -656,7 +694,6 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
   }
   if (act) {
     wv_st(V.ph, V.W, i, ph);
-    wv_st(V.ex, V.W, i, ex);
     if (G > 0)
       L_ROLL
       for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = dw[p];
@@ -870,16 +907,18 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
   int W = (int)((want + 255) / 256 * 256);
   const size_t nph = (pk.nav64 ? sizeof(PhotonT<double>) : sizeof(Photon)) / 4, nex = sizeof(WaveExtra) / 4;
   const size_t npre = (pk.nav64 ? sizeof(PreT<double>) : sizeof(Pre)) / 4;
-  const size_t nq = (pk.nav64 ? sizeof(QueryT<double>) : sizeof(Query)) / 4;
+  const size_t nq = (pk.nav64 ? sizeof(WaveQuery<double>) : sizeof(WaveQuery<float>)) / 4;
+  const size_t npt = sizeof(PhotonTally) / 4;
   const size_t ng = G > 0 ? LUMEN_MAX_GRAD : 0;
-  size_t words = (size_t)W * (nph + nex + npre + nq + ng + 3) + 2;
+  size_t words = (size_t)W * (nph + nex + npt + npre + nq + ng + 3) + 2;
   uint32_t* buf = nullptr;
   CK(cudaMallocAsync((void**)&buf, words * 4, stream));
   Wave V;
   V.W = W;
   V.ph = buf;
   V.ex = V.ph + (size_t)W * nph;
-  V.pre = V.ex + (size_t)W * nex;
+  V.pt = V.ex + (size_t)W * nex;
+  V.pre = V.pt + (size_t)W * npt;
   V.q = V.pre + (size_t)W * npre;
   V.dw = (float*)(V.q + (size_t)W * nq);
   int32_t* list[2] = {(int32_t*)(V.dw + (size_t)W * ng), (int32_t*)(V.dw + (size_t)W * ng) + W};
@@ -942,6 +981,7 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     Launch LD = L;
     LD.wv_ph = V.ph;
     LD.wv_ex = V.ex;
+    LD.wv_pt = V.pt;
     LD.wv_dw = V.dw;
     LD.wv_list = V.out;
     LD.wv_n = V.n_out;
