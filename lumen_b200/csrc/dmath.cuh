@@ -271,10 +271,42 @@ L_DEV Key fold_in(Key k, uint32_t d) {
   return r;
 }
 
+L_DEV float uniform_of(uint32_t y0, uint32_t y1) {
+  uint32_t b = (y0 ^ y1) >> 9;
+  return ((float)b + 0.5f) * 1.1920928955078125e-7f;
+}
 L_DEV float uniform(Key k, uint32_t i) {
   const uint2 y = threefry(k.k0, k.k1, 0u, i);
-  uint32_t b = (y.x ^ y.y) >> 9;
-  return ((float)b + 0.5f) * 1.1920928955078125e-7f;
+  return uniform_of(y.x, y.y);
+}
+
+// N blocks side by side, the same words as one by one: a block is a chain of some 65 dependent operations. Where a walk
+// draws five in turn they are its longest link (below); three draws at once for a lobe or a facet cost the step with
+// tangents 9 % (registers held over the call) and gave the others nothing.
+template <int N>
+L_DEV void threefry_n(const uint32_t* k0, const uint32_t* k1, uint32_t* x0, uint32_t* x1) {
+  uint32_t k2[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) { k2[j] = k0[j] ^ k1[j] ^ 0x1BD11BDAu; x0[j] += k0[j]; x1[j] += k1[j]; }
+#define TF_R(r) _Pragma("unroll") for (int j = 0; j < N; ++j) { x0[j] += x1[j]; x1[j] = rotl(x1[j], r); x1[j] ^= x0[j]; }
+#define TF_K(a, b, c) _Pragma("unroll") for (int j = 0; j < N; ++j) { x0[j] += a[j]; x1[j] += b[j] + c; }
+  TF_R(13) TF_R(15) TF_R(26) TF_R(6) TF_K(k1, k2, 1u)
+  TF_R(17) TF_R(29) TF_R(16) TF_R(24) TF_K(k2, k0, 2u)
+  TF_R(13) TF_R(15) TF_R(26) TF_R(6) TF_K(k0, k1, 3u)
+  TF_R(17) TF_R(29) TF_R(16) TF_R(24) TF_K(k1, k2, 4u)
+  TF_R(13) TF_R(15) TF_R(26) TF_R(6) TF_K(k2, k0, 5u)
+#undef TF_K
+#undef TF_R
+}
+// a key's uniforms 0 to 3, and another key's fold by d (the walk's next scattering)
+struct Draws { float u0, u1, u2, u3; Key next; };
+L_CALL Draws uniform4_fold(Key k, Key f, uint32_t d) {
+  uint32_t k0[5] = {k.k0, k.k0, k.k0, k.k0, f.k0}, k1[5] = {k.k1, k.k1, k.k1, k.k1, f.k1};
+  uint32_t x0[5] = {0u, 0u, 0u, 0u, 0u}, x1[5] = {0u, 1u, 2u, 3u, d};
+  threefry_n<5>(k0, k1, x0, x1);
+  Draws r = {uniform_of(x0[0], x1[0]), uniform_of(x0[1], x1[1]), uniform_of(x0[2], x1[2]), uniform_of(x0[3], x1[3]),
+             {x0[4], x1[4]}};
+  return r;
 }
 
 }  // namespace lb

@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
   unsigned c_ph = 0, c_steps = 0, c_dep = 0, c_trunc = 0, c_multi = 0, c_lost = 0;
   int budget_chunk = 0;
   if constexpr (!ANALOG) {
-    const unsigned t = blockIdx.x * BLOCK + threadIdx.x;
+    // the first warps of all blocks, then the second: few slots spread over every SM
+    const unsigned t = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + lane;
     if (L.wv_W > 0 && t < *L.wv_n) {  // a wavefront slot's photon, where its last round left it
       const int i = L.wv_list[t];
       WaveExtra ex;
@@ -845,7 +846,13 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 // persistent loop resumes every slot still live (one thread a slot) and takes the photons left. Each round's query
 // writes its live slots to page-locked host memory as it starts (`pub`), and a synchronous call launches round r once
 // it has seen round r - LUMEN_WAVE_AHEAD's: no round waits for the host, the grids follow the live slots down (they
-// only ever fall), and the drain starts once fewer than a 64th of the slots are live. An asynchronous call
+// only ever fall), and the drain starts once fewer than a 64th of the slots, or than LUMEN_WAVE_MIN, are live: a round is
+// two launches that wait for their slowest photon, and below some 8192 photons, 2 warps a scheduler, that wait is all
+// there is (a call of fewer photons runs the persistent loop from the start). Drain below a 64th, 2048, 4096, 8192,
+// 16384, same box, ms: liquid-argon box 21.5, 21.2, 20.7, 20.2, 20.7; solids box 8.1, 8.2, 7.8, 7.6, 7.2; fog box 9.4,
+// 8.7, 8.2, 8.1, 8.8; the others within 1 %. The whole call, persistent loop against wavefront, at 1024, 4096-8192 and
+// 16384 photons: tank 0.57 / 1.12, -, 0.72 / 0.74; liquid-argon box -, 9.8 / 13.3, 26 / 15; solids box 2.9 / 4.5,
+// 4.6 / 5.7, -; fog box 4.0 / 6.5, -, 8.9 / 8.2; toy tank -, 0.42 / 0.46, 0.47 / 0.47 (32768). An asynchronous call
 // (LUMEN_F_ASYNC) runs `rounds` rounds over the whole pool without a readback (<= 0: *rpp rounds per photon a slot
 // carries, the scene's estimate from its last synchronous call) and drains. Against rounds over the whole pool with a
 // readback every fourth (2^24 photons of the tank 45.5 -> 43.6 ms, 1,000,003 5.08 -> 3.83, the ground-wall tank with
@@ -855,6 +862,7 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 // (about 360 bytes each with gradients), allocated on the call's stream.
 #define LUMEN_WAVE_POOL (1 << 21)
 #define LUMEN_WAVE_AHEAD 2
+#define LUMEN_WAVE_MIN 8192
 
 // threads a block for n live slots: whole blocks of 256 while they fill the chip several times over, fewer where that
 // leaves SMs without one (148 SMs)
@@ -953,7 +961,7 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
         CK(cudaStreamSynchronize(stream));
         return set_err(LUMEN_ERR_CUDA, "the wavefront's rounds ended early");
       }
-      if (live < W / 64) break;
+      if (live < std::max(W / 64, LUMEN_WAVE_MIN)) break;
     }
     std::swap(list[0], list[1]);
     V.in = list[1];
@@ -986,7 +994,9 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     LD.wv_list = V.out;
     LD.wv_n = V.n_out;
     LD.wv_W = W;
-    const int grid = (int)(((async ? W : live) + 255) / 256);
+    // one thread a slot, over as many SMs as there are warps of them
+    const long long most = async ? W : live;
+    const int grid = (int)std::max((most + 255) / 256, std::min((most + 31) / 32, 148LL));
     if (pk.nav64)
       st = pk.single ? launch_shape<G, 256, 4, 2, 0, 1>(LD, 0, stream, grid)
                      : (pk.groups ? launch_shape<G, 256, 4, 3, 0, 1>(LD, 0, stream, grid)

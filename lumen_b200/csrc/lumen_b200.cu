@@ -662,6 +662,7 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
     L.truth = out->truth;
     if (variant == LUMEN_VARIANT_WAVEFRONT) variant = 0;
   }
+  if (variant == LUMEN_VARIANT_WAVEFRONT && !async && L.n < LUMEN_WAVE_MIN) variant = 0;  // run_wave's drain alone
   if (variant == LUMEN_VARIANT_WAVEFRONT && !async)
     if (int st = pub.take()) return st;
   T.grads = grads;
