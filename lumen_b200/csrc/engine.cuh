@@ -46,6 +46,7 @@ struct LumenScene {
   int single;                          // every solid one quadric / plane leaf: the single-leaf instantiation
   int clip;                            // the extended locate is needed: a protrusion clip or frame groups
   int groups;                          // frame groups (the instantiation walking them)
+  int lobes;                           // a row draws facets, or a medium has a Mie or WLS channel
   int nav64;                           // LUMEN_PREC_FLOAT64: S's vol_f, node_f, leaf_f, plane_f hold float64 data
   const float* vol_f32;                // the float32 frames (the readout groups' binning reads them in either precision)
   // the wavefront's rounds per photon a slot carries, from the last synchronous wavefront call (an estimate for the
@@ -155,6 +156,7 @@ struct Pick {
   int groups;              // frame groups: the extended instantiation with their traversal
   int analog;
   int nav64;               // the scene's navigator is float64
+  int lobes;               // a row draws facets, or a medium has a Mie or WLS channel
   int born;                // a sensor counts the photons born inside it (the wavefront's step kernel with that branch)
   const float* vol_f32;    // the scene's float32 frames (the readout binning)
 };
@@ -287,6 +289,7 @@ struct WaveQuery {
   int vol_at, srf;
 };
 
+#define LUMEN_STEP_BLOCK 512  // the step kernel's largest block (its registers allow an SM 512 threads)
 struct Wave {  // the records of the navigator's precision NF
   uint32_t* ph;     // W x sizeof(PhotonT<NF>) / 4
   uint32_t* ex;     // W x sizeof(WaveExtra) / 4
@@ -296,7 +299,7 @@ struct Wave {  // the records of the navigator's precision NF
   float* dw;        // W x LUMEN_MAX_GRAD (gradient runs)
   int W;
   // the round's live slots in[0, *n_in) and the next round's out[0, *n_out); mid: the same slots after the query, each
-  // block's photons that scatter before their crossing ahead of its others (slot | place in the block's list << 24)
+  // block's photons that scatter before their crossing ahead of its others (slot | place in the list mod 512 << 23)
   const int32_t* in;
   const unsigned* n_in;
   int32_t* out;
@@ -585,7 +588,7 @@ __global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wav
   }
   if (in) {
     const unsigned at = bulk ? before : all + threadIdx.x - before;
-    V.mid[blockIdx.x * blockDim.x + at] = (uint32_t)i | (threadIdx.x << 24);
+    V.mid[blockIdx.x * blockDim.x + at] = (uint32_t)i | ((j & 511u) << 23);
   }
 }
 
@@ -593,24 +596,24 @@ __global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wav
 // none of the query the query kernel made for it; a scene without one runs the kernel compiled without the branch,
 // the branch costs the tank's plain forward 2 % where it is compiled in)
 template <int G, int BORN, int EXT, int NAV64>
-__global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
+__global__ void __launch_bounds__(LUMEN_STEP_BLOCK, 512 / LUMEN_STEP_BLOCK) k_wave_step(Launch L, Wave V) {
   using NF = typename NavOf<NAV64>::F;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   __shared__ double sh_health[LUMEN_N_HEALTH];
-  __shared__ unsigned long long sc[LUMEN_N_COUNT][8];
-  __shared__ unsigned on[8], base_out;
+  __shared__ unsigned long long sc[LUMEN_N_COUNT][LUMEN_STEP_BLOCK / 32];
+  __shared__ unsigned on[16], base_out;
   const unsigned n = *V.n_in;
   const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (blockIdx.x * blockDim.x >= n) return;
   if (threadIdx.x < LUMEN_N_HEALTH) sh_health[threadIdx.x] = 0.0;
-  if (threadIdx.x < 8) on[threadIdx.x] = 0u;
+  if (threadIdx.x < 16) on[threadIdx.x] = 0u;
   __syncthreads();
   const int in = j < n;
   const int aborted = L.abort_flag && *(volatile int*)L.abort_flag;
   int act = in && !aborted;
   const uint32_t mid = act ? V.mid[j] : 0u;
-  const int i = (int)(mid & 0xffffffu);
+  const int i = (int)(mid & 0x7fffffu);
   unsigned c_ph = 0, c_steps = 0, c_dep = 0, c_trunc = 0, c_multi = 0, c_lost = 0;
   PhotonT<NF> ph;
   WaveExtra ex;
@@ -700,12 +703,12 @@ __global__ void __launch_bounds__(256, 2) k_wave_step(Launch L, Wave V) {
       for (int p = 0; p < L.R.P; ++p) V.dw[(size_t)p * V.W + i] = dw[p];
   }
   // the next round's list: the block's slots that go on, in the order they came in, one atomic a block
-  const unsigned place = mid >> 24;
+  const unsigned place = mid >> 23;
   if (act) atomicOr(&on[place >> 5], 1u << (place & 31u));
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned sum = 0;
-    for (int w = 0; w < 8; ++w) sum += __popc(on[w]);
+    for (int w = 0; w < 16; ++w) sum += __popc(on[w]);
     base_out = sum ? atomicAdd(V.n_out, sum) : 0u;
   }
   __syncthreads();
@@ -865,7 +868,11 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 #define LUMEN_WAVE_MIN 8192
 
 // threads a block for n live slots: whole blocks of 256 while they fill the chip several times over, fewer where that
-// leaves SMs without one (148 SMs)
+// leaves SMs without one (148 SMs). Large blocks are the better ones: their warps start together and share the
+// instruction fetch that the step waits on (step blocks of 256, 128, 64, 32, same box, ms: tank 2^24 photons 35.2, 40.5,
+// 44.0, 46.6; ground wall with four tangents 9.8, 10.9, 11.6, 11.9; readout tank 7.6, 8.9, 9.3, 9.5). Where the step's
+// code is longest, in scenes that draw facets or have a Mie or WLS channel, it runs in blocks of 512, one an SM (ground
+// wall 9.85 -> 8.98, readout tank 7.63 -> 6.79; the polished tank's 1,000,003 photons lose 1 % in them)
 inline int wave_block(unsigned n) { return n >= 148u * 256u * 4u ? 256 : (n >= 148u * 128u * 2u ? 128 : (n >= 148u * 64u ? 64 : 32)); }
 
 // waits for a published round >= `want`; returns its live slots, or -1 where the stream failed
@@ -970,6 +977,7 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     V.n_out = cnt + ((r + 1) & 1);
     V.round = (unsigned)r;
     const int block = wave_block((unsigned)live), grid = (int)((live + block - 1) / block);
+    const int sblock = block == 256 && pk.lobes ? LUMEN_STEP_BLOCK : block, sgrid = (int)((live + sblock - 1) / sblock);
     if (pk.nav64)
       st = pk.single ? launch_wave_query<2, 1>(L, V, grid, block, stream)
                      : (pk.groups ? launch_wave_query<3, 1>(L, V, grid, block, stream)
@@ -979,10 +987,10 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     else if (pk.single) st = launch_wave_query<2, 0>(L, V, grid, block, stream);
     else st = launch_wave_query<0, 0>(L, V, grid, block, stream);
     if (st) return st;
-    if (pk.nav64) st = launch_wave_step<G, 1, 1, 1>(L, V, grid, block, stream);
-    else if (pk.born) st = launch_wave_step<G, 1, 1, 0>(L, V, grid, block, stream);
-    else if (ext) st = launch_wave_step<G, 0, 1, 0>(L, V, grid, block, stream);
-    else st = launch_wave_step<G, 0, 0, 0>(L, V, grid, block, stream);
+    if (pk.nav64) st = launch_wave_step<G, 1, 1, 1>(L, V, sgrid, sblock, stream);
+    else if (pk.born) st = launch_wave_step<G, 1, 1, 0>(L, V, sgrid, sblock, stream);
+    else if (ext) st = launch_wave_step<G, 0, 1, 0>(L, V, sgrid, sblock, stream);
+    else st = launch_wave_step<G, 0, 0, 0>(L, V, sgrid, sblock, stream);
     if (st) return st;
   }
   if (live > 0) {  // the persistent loop finishes the live slots and takes the photons left

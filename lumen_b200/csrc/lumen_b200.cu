@@ -536,6 +536,7 @@ static int fill_launch(const LumenScene* sc, const LumenRows* rows, const LumenS
   pk.clip = sc->clip;
   pk.groups = sc->groups;
   pk.nav64 = sc->nav64;
+  pk.lobes = sc->lobes;
   pk.born = sc->S.cls_born != nullptr;
   pk.vol_f32 = sc->vol_f32;
   pk.analog = (c->flags & LUMEN_F_TRUTH) != 0;
@@ -1046,6 +1047,7 @@ int32_t lumen_b200_scene_create(const LumenSceneDesc* d, LumenScene** out) {
     const int32_t* ri = d->row_i + r * LUMEN_ROW_I;
     if (ri[LUMEN_RI_MODEL] == 0 && !ri[LUMEN_RI_NORMAL] && !ri[LUMEN_RI_GLISUR])
       sc->sigma_tabs.push_back(ri[LUMEN_RI_COL + LUMEN_COL_SIGMA]);
+    sc->lobes = sc->lobes || ri[LUMEN_RI_GLISUR] || (ri[LUMEN_RI_MODEL] == 0 && !ri[LUMEN_RI_NORMAL]);
   }
   sc->tab.assign(d->tab, d->tab + 2 * (size_t)d->n_tab);
   sc->has_torus = d->n_mesh > 0 || d->n_group > 0;  // the extended instantiation: tori, meshes, frame groups
@@ -1065,6 +1067,7 @@ int32_t lumen_b200_scene_create(const LumenSceneDesc* d, LumenScene** out) {
   for (int m = 0; m < d->n_med; ++m) {
     const int32_t* mr = d->med_i + (size_t)m * LUMEN_MED_I;
     if (mr[LUMEN_MI_WLS] >= 0) sc->spectrum_tabs.push_back(mr[LUMEN_MI_WLS_SPEC]);
+    sc->lobes = sc->lobes || mr[LUMEN_MI_WLS] >= 0 || mr[LUMEN_MI_MIE] >= 0;
   }
   value_roles(d, sc->roles);
   if (check_widths(sc, d->pool)) {

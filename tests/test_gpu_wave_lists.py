@@ -76,6 +76,13 @@ def test_tangents_with_clips_and_float64():
         _agree(_run(eng, name, 9001, grads, variant=A.VARIANT_WAVEFRONT), _run(eng, name, 9001, grads, variant=0))
 
 
+@pytest.mark.parametrize("name,grads", [("readout_tank", ()), ("protrusion_box", ()), ("mesh_tank", ("surfaces/Wall/R",))])
+def test_largest_blocks(name, grads):
+    """Enough live slots for the step's blocks of 512 (scenes with facets), the last one ragged; fewer as they end."""
+    eng = _engine(name, "float32")
+    _agree(_run(eng, name, 152001, grads, variant=A.VARIANT_WAVEFRONT), _run(eng, name, 152001, grads, variant=0))
+
+
 def test_step_budget_ends_the_rounds():
     eng = _engine("lar_box", "float32")
     src = sources.Point(position=AT["lar_box"], n_photons=1.0, lam=420.0)
