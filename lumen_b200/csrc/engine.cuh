@@ -56,12 +56,14 @@ struct LumenScene {
   // the scene's later calls (as many as have run at once) and freed with it
   mutable std::mutex pub_mu;
   mutable std::vector<unsigned long long*> pub_free;
+  mutable std::vector<unsigned long long*> pub_left;  // of calls that ended in an error: kernels may still write them
 };
 
 // one of the scene's published words for the length of a call
 struct PubLease {
   const LumenScene* sc;
   unsigned long long* p = nullptr;
+  int idle = 0;  // the call has waited for its stream: nothing writes the word any more
   explicit PubLease(const LumenScene* s) : sc(s) {}
   int take() {
     {
@@ -75,10 +77,10 @@ struct PubLease {
     CK(cudaHostAlloc((void**)&p, sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped));
     return 0;
   }
-  ~PubLease() {  // every path out of a synchronous call has waited for its stream, or left an error on it
+  ~PubLease() {
     if (!p) return;
     std::lock_guard<std::mutex> lock(sc->pub_mu);
-    sc->pub_free.push_back(p);
+    (idle ? sc->pub_free : sc->pub_left).push_back(p);
   }
 };
 

@@ -158,7 +158,10 @@ struct RayTree {
     while (((long long)1 << (l - 1)) < m) ++l;
     return l;
   }
-  double centre(int i, int ax) const { return 0.5 * ((double)box[i].v[ax] + box[i].v[3 + ax]); }
+  double centre(int i, int ax) const {
+    const double c = 0.5 * ((double)box[i].v[ax] + box[i].v[3 + ax]);
+    return c == c ? c : 0.0;  // (-inf, inf)
+  }
   void order(int a, int b, int ax) {
     std::sort(id.begin() + a, id.begin() + b, [&](int p, int q) {
       const double cp = centre(p, ax), cq = centre(q, ax);
@@ -240,6 +243,11 @@ static void ray_records(const LumenSceneDesc* d, std::vector<float>& rec, std::v
       }
       RayTree::Box b;
       memcpy(b.v, d->node_f + (size_t)nd * LUMEN_NODE_F, sizeof(b.v));
+      for (int k = 0; k < 6; ++k)
+        if (b.v[k] != b.v[k]) {  // a box with a NaN meets no ray (as every comparison with it): one out of every ray's reach
+          std::fill(b.v, b.v + 6, 3e38f);
+          break;
+        }
       t.id.push_back((int)t.box.size());
       t.box.push_back(b);
       t.weight.push_back(ni[1]);
@@ -759,6 +767,7 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
   CK(cudaFreeAsync(scratch, stream));
   if (dummy) CK(cudaFreeAsync(dummy, stream));
   CK(cudaStreamSynchronize(stream));
+  pub.idle = 1;
   if (flag) return set_err(LUMEN_ERR_STEP_BUDGET, "the call's step budget ran out before every photon ended");
   if (groups && n_rec > (unsigned long long)out->rec_capacity)
     return set_err(LUMEN_ERR_RECORDS, "the deposit records outgrew rec_capacity (" + std::to_string(n_rec) +
@@ -1110,6 +1119,7 @@ int32_t lumen_b200_scene_destroy(LumenScene* sc) {
   if (!sc) return 0;
   for (void* p : sc->allocs) cudaFree(p);
   for (unsigned long long* p : sc->pub_free) cudaFreeHost(p);
+  for (unsigned long long* p : sc->pub_left) cudaFreeHost(p);
   delete sc;
   return 0;
 }
