@@ -291,7 +291,11 @@ struct WaveQuery {
   int vol_at, srf;
 };
 
+#define LUMEN_QUERY_BLOCK(nav64) ((nav64) ? 512 : 768)  // the query kernel's largest block: an SM's threads by its registers
 #define LUMEN_STEP_BLOCK 512  // the step kernel's largest block (its registers allow an SM 512 threads)
+#ifndef QSEL
+#define QSEL LUMEN_QUERY_BLOCK(pk.nav64)
+#endif
 struct Wave {  // the records of the navigator's precision NF
   uint32_t* ph;     // W x sizeof(PhotonT<NF>) / 4
   uint32_t* ex;     // W x sizeof(WaveExtra) / 4
@@ -548,9 +552,9 @@ __global__ void __launch_bounds__(256) k_wave_fill(Launch L, Wave V) {
 }
 
 template <int TORUS, int NAV64>
-__global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wave V) {
+__global__ void __launch_bounds__(LUMEN_QUERY_BLOCK(NAV64), 1) k_wave_query(Launch L, Wave V) {
   using NF = typename NavOf<NAV64>::F;
-  __shared__ unsigned sh[8];
+  __shared__ unsigned sh[24];
   const unsigned n = *V.n_in;
   const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j == 0) {
@@ -583,14 +587,17 @@ __global__ void __launch_bounds__(256, NAV64 ? 2 : 3) k_wave_query(Launch L, Wav
   const unsigned m = __ballot_sync(0xffffffffu, in && bulk);
   if (lane == 0) sh[warp] = __popc(m);
   __syncthreads();
-  unsigned before = __popc(m & ((1u << lane) - 1u)), all = 0;  // the block's scatterings ahead of this thread, and all
-  for (int w = 0; w < warps; ++w) {
+  // the scatterings ahead of this thread, and all, of its 256 threads (a larger block orders each 256 by themselves: the
+  // step's blocks hold whole ones)
+  const int w0 = warp & ~7;
+  unsigned before = __popc(m & ((1u << lane) - 1u)), all = 0;
+  for (int w = w0; w < w0 + 8 && w < warps; ++w) {
     if (w < warp) before += sh[w];
     all += sh[w];
   }
   if (in) {
-    const unsigned at = bulk ? before : all + threadIdx.x - before;
-    V.mid[blockIdx.x * blockDim.x + at] = (uint32_t)i | ((j & 511u) << 23);
+    const unsigned at = bulk ? before : all + (threadIdx.x & 255u) - before;
+    V.mid[blockIdx.x * blockDim.x + (threadIdx.x & ~255u) + at] = (uint32_t)i | ((j & 511u) << 23);
   }
 }
 
@@ -979,15 +986,16 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     V.n_out = cnt + ((r + 1) & 1);
     V.round = (unsigned)r;
     const int block = wave_block((unsigned)live), grid = (int)((live + block - 1) / block);
+    const int qblock = block == 256 ? (QSEL) : block, qgrid = (int)((live + qblock - 1) / qblock);
     const int sblock = block == 256 && pk.lobes ? LUMEN_STEP_BLOCK : block, sgrid = (int)((live + sblock - 1) / sblock);
     if (pk.nav64)
-      st = pk.single ? launch_wave_query<2, 1>(L, V, grid, block, stream)
-                     : (pk.groups ? launch_wave_query<3, 1>(L, V, grid, block, stream)
-                                  : launch_wave_query<1, 1>(L, V, grid, block, stream));
-    else if (pk.groups) st = launch_wave_query<3, 0>(L, V, grid, block, stream);
-    else if (pk.torus) st = launch_wave_query<1, 0>(L, V, grid, block, stream);
-    else if (pk.single) st = launch_wave_query<2, 0>(L, V, grid, block, stream);
-    else st = launch_wave_query<0, 0>(L, V, grid, block, stream);
+      st = pk.single ? launch_wave_query<2, 1>(L, V, qgrid, qblock, stream)
+                     : (pk.groups ? launch_wave_query<3, 1>(L, V, qgrid, qblock, stream)
+                                  : launch_wave_query<1, 1>(L, V, qgrid, qblock, stream));
+    else if (pk.groups) st = launch_wave_query<3, 0>(L, V, qgrid, qblock, stream);
+    else if (pk.torus) st = launch_wave_query<1, 0>(L, V, qgrid, qblock, stream);
+    else if (pk.single) st = launch_wave_query<2, 0>(L, V, qgrid, qblock, stream);
+    else st = launch_wave_query<0, 0>(L, V, qgrid, qblock, stream);
     if (st) return st;
     if (pk.nav64) st = launch_wave_step<G, 1, 1, 1>(L, V, sgrid, sblock, stream);
     else if (pk.born) st = launch_wave_step<G, 1, 1, 0>(L, V, sgrid, sblock, stream);
