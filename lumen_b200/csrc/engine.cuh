@@ -291,11 +291,13 @@ struct WaveQuery {
   int vol_at, srf;
 };
 
-#define LUMEN_QUERY_BLOCK(nav64) ((nav64) ? 512 : 768)  // the query kernel's largest block: an SM's threads by its registers
+// the query kernel's largest block, 3 an SM (2 in float64): the wait of a block for its slowest warp grows with it (blocks
+// of 256, 384, 512 and 768, same box, ms: tank 2^24 photons 35.0, 35.3, 40.4, 36.7; 1,000,003 2.89, 2.93, 3.18, 3.04; track
+// events 11.5, 11.7, 12.7, 11.9; ground wall with four tangents 8.97, 9.20, 9.64, 9.22; float64 panel 256 and 512 3.22, 3.27)
+#define LUMEN_QUERY_BLOCK 256
 #define LUMEN_STEP_BLOCK 512  // the step kernel's largest block (its registers allow an SM 512 threads)
-#ifndef QSEL
-#define QSEL LUMEN_QUERY_BLOCK(pk.nav64)
-#endif
+// a slot's place in its step block is 9 bits of `mid`, and every block of the step holds whole blocks of the query
+static_assert(LUMEN_STEP_BLOCK <= 512 && LUMEN_STEP_BLOCK % LUMEN_QUERY_BLOCK == 0, "a step block's places");
 struct Wave {  // the records of the navigator's precision NF
   uint32_t* ph;     // W x sizeof(PhotonT<NF>) / 4
   uint32_t* ex;     // W x sizeof(WaveExtra) / 4
@@ -552,9 +554,9 @@ __global__ void __launch_bounds__(256) k_wave_fill(Launch L, Wave V) {
 }
 
 template <int TORUS, int NAV64>
-__global__ void __launch_bounds__(LUMEN_QUERY_BLOCK(NAV64), 1) k_wave_query(Launch L, Wave V) {
+__global__ void __launch_bounds__(LUMEN_QUERY_BLOCK, NAV64 ? 2 : 3) k_wave_query(Launch L, Wave V) {
   using NF = typename NavOf<NAV64>::F;
-  __shared__ unsigned sh[24];
+  __shared__ unsigned sh[LUMEN_QUERY_BLOCK / 32];
   const unsigned n = *V.n_in;
   const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j == 0) {
@@ -587,17 +589,15 @@ __global__ void __launch_bounds__(LUMEN_QUERY_BLOCK(NAV64), 1) k_wave_query(Laun
   const unsigned m = __ballot_sync(0xffffffffu, in && bulk);
   if (lane == 0) sh[warp] = __popc(m);
   __syncthreads();
-  // the scatterings ahead of this thread, and all, of its 256 threads (a larger block orders each 256 by themselves: the
-  // step's blocks hold whole ones)
-  const int w0 = warp & ~7;
+  // the scatterings ahead of this thread, and all of the block's
   unsigned before = __popc(m & ((1u << lane) - 1u)), all = 0;
-  for (int w = w0; w < w0 + 8 && w < warps; ++w) {
+  for (int w = 0; w < warps; ++w) {
     if (w < warp) before += sh[w];
     all += sh[w];
   }
   if (in) {
-    const unsigned at = bulk ? before : all + (threadIdx.x & 255u) - before;
-    V.mid[blockIdx.x * blockDim.x + (threadIdx.x & ~255u) + at] = (uint32_t)i | ((j & 511u) << 23);
+    const unsigned at = bulk ? before : all + threadIdx.x - before;
+    V.mid[blockIdx.x * blockDim.x + at] = (uint32_t)i | ((j & 511u) << 23);
   }
 }
 
@@ -882,7 +882,7 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 // 44.0, 46.6; ground wall with four tangents 9.8, 10.9, 11.6, 11.9; readout tank 7.6, 8.9, 9.3, 9.5). Where the step's
 // code is longest, in scenes that draw facets or have a Mie or WLS channel, it runs in blocks of 512, one an SM (ground
 // wall 9.85 -> 8.98, readout tank 7.63 -> 6.79; the polished tank's 1,000,003 photons lose 1 % in them)
-inline int wave_block(unsigned n) { return n >= 148u * 256u * 4u ? 256 : (n >= 148u * 128u * 2u ? 128 : (n >= 148u * 64u ? 64 : 32)); }
+inline int wave_block(unsigned n) { return n >= 148u * 256u * 4u ? LUMEN_QUERY_BLOCK : (n >= 148u * 128u * 2u ? 128 : (n >= 148u * 64u ? 64 : 32)); }
 
 // waits for a published round >= `want`; returns its live slots, or -1 where the stream failed
 inline long long wave_seen(volatile unsigned long long* pub, long long want, cudaStream_t stream) {
@@ -986,16 +986,15 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
     V.n_out = cnt + ((r + 1) & 1);
     V.round = (unsigned)r;
     const int block = wave_block((unsigned)live), grid = (int)((live + block - 1) / block);
-    const int qblock = block == 256 ? (QSEL) : block, qgrid = (int)((live + qblock - 1) / qblock);
-    const int sblock = block == 256 && pk.lobes ? LUMEN_STEP_BLOCK : block, sgrid = (int)((live + sblock - 1) / sblock);
+    const int sblock = block == LUMEN_QUERY_BLOCK && pk.lobes ? LUMEN_STEP_BLOCK : block, sgrid = (int)((live + sblock - 1) / sblock);
     if (pk.nav64)
-      st = pk.single ? launch_wave_query<2, 1>(L, V, qgrid, qblock, stream)
-                     : (pk.groups ? launch_wave_query<3, 1>(L, V, qgrid, qblock, stream)
-                                  : launch_wave_query<1, 1>(L, V, qgrid, qblock, stream));
-    else if (pk.groups) st = launch_wave_query<3, 0>(L, V, qgrid, qblock, stream);
-    else if (pk.torus) st = launch_wave_query<1, 0>(L, V, qgrid, qblock, stream);
-    else if (pk.single) st = launch_wave_query<2, 0>(L, V, qgrid, qblock, stream);
-    else st = launch_wave_query<0, 0>(L, V, qgrid, qblock, stream);
+      st = pk.single ? launch_wave_query<2, 1>(L, V, grid, block, stream)
+                     : (pk.groups ? launch_wave_query<3, 1>(L, V, grid, block, stream)
+                                  : launch_wave_query<1, 1>(L, V, grid, block, stream));
+    else if (pk.groups) st = launch_wave_query<3, 0>(L, V, grid, block, stream);
+    else if (pk.torus) st = launch_wave_query<1, 0>(L, V, grid, block, stream);
+    else if (pk.single) st = launch_wave_query<2, 0>(L, V, grid, block, stream);
+    else st = launch_wave_query<0, 0>(L, V, grid, block, stream);
     if (st) return st;
     if (pk.nav64) st = launch_wave_step<G, 1, 1, 1>(L, V, sgrid, sblock, stream);
     else if (pk.born) st = launch_wave_step<G, 1, 1, 0>(L, V, sgrid, sblock, stream);
