@@ -110,3 +110,26 @@ def test_two_rank_sharding_equals_one_process():
         np.testing.assert_allclose(jac, want[4], rtol=1e-9, atol=1e-15)
         assert photons == N and steps == int(T.counts[A.C_STEPS])
         assert a_surf == pytest.approx(T.health[5], rel=1e-9)
+
+
+def test_results_of_a_tracer_with_tallies_of_its_own():
+    """A tracer may hand back its own tallies in place of the ones it was given (the arrays all_reduce_tallies adds)."""
+    from types import SimpleNamespace
+
+    from lumen_b200 import detectors, distributed, sources
+
+    det = detectors.toy_tank()
+    src = sources.Point(position=(0.05, 0.02, 0.1), n_photons=1.0, lam=420.0)
+    given = _checker_tracer(det, src, 512)
+
+    def own(first, n, key, controls, T):
+        T = given(first, n, key, controls, T)
+        return SimpleNamespace(**{k: None if getattr(T, k) is None else getattr(T, k).clone() for k in (
+            "arrival", "arrival_t", "arrival2", "hist", "jac", "health", "counts")})  # fmt: skip
+
+    want = distributed.simulate_sharded(det, src, samples=512, seed=1, time_bins=(4, 0.0, 1.0), tracer=given)
+    got = distributed.simulate_sharded(det, src, samples=512, seed=1, time_bins=(4, 0.0, 1.0), tracer=own)
+    for k in ("arrivals", "arrivals_error", "mean_arrival_time"):
+        np.testing.assert_array_equal(getattr(got, k), getattr(want, k))
+    np.testing.assert_array_equal(got.diagnostics["time"], want.diagnostics["time"])
+    assert got.health == want.health

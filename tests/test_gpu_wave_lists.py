@@ -122,3 +122,22 @@ def test_results_are_numpys(events, sensors, bins, grads):
     np.testing.assert_array_equal(T.arrival2.cpu().numpy(), error)
     np.testing.assert_array_equal(T.arrival_t.cpu().numpy(), time)
     assert int(T.nonfinite.item()) == want_bad
+
+
+def test_results_of_a_tracer_on_the_device():
+    """simulate_sharded with a caller's tracer whose tallies are on the GPU: the results of the engine's own share."""
+    from lumen_b200 import distributed
+
+    eng = _engine("toy_tank", "float32")
+    det, src = eng.det, sources.Point(position=AT["toy_tank"], n_photons=1.0, lam=420.0)
+
+    def tracer(first, n, key, controls, T):
+        T = DeviceTallies(T.arrival.shape[1], T.arrival.shape[0], 0, 0.0, 1.0, 0)
+        eng.trace(key, n, source=DeviceSource(src, 4099, det=det), first_id=first, controls=controls, tallies=T)
+        return T
+
+    want = distributed.simulate_sharded(det, src, samples=4099, seed=3)
+    got = distributed.simulate_sharded(det, src, samples=4099, seed=3, tracer=tracer)
+    for k in ("arrivals", "arrivals_error", "mean_arrival_time"):
+        np.testing.assert_allclose(getattr(got, k), getattr(want, k), rtol=1e-9, atol=1e-12)
+    assert got.health.photons == 4099
