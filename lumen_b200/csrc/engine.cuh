@@ -56,29 +56,31 @@ struct LumenScene {
   // the scene's later calls (as many as have run at once) and freed with it
   mutable std::mutex pub_mu;
   mutable std::vector<unsigned long long*> pub_free;
-  mutable std::vector<unsigned long long*> pub_left;  // of calls that ended in an error: kernels may still write them
+  mutable std::vector<unsigned long long*> pub_left;  // of calls whose stream failed: kernels may still write them
 };
 
-// one of the scene's published words for the length of a call
+// one of the scene's published words, from the launch of the rounds that write it to the end of the call
 struct PubLease {
   const LumenScene* sc;
+  cudaStream_t stream;
   unsigned long long* p = nullptr;
   int idle = 0;  // the call has waited for its stream: nothing writes the word any more
-  explicit PubLease(const LumenScene* s) : sc(s) {}
+  PubLease(const LumenScene* s, cudaStream_t st) : sc(s), stream(st) {}
   int take() {
     {
       std::lock_guard<std::mutex> lock(sc->pub_mu);
       if (!sc->pub_free.empty()) {
         p = sc->pub_free.back();
         sc->pub_free.pop_back();
-        return 0;
       }
     }
-    CK(cudaHostAlloc((void**)&p, sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped));
+    if (!p) CK(cudaHostAlloc((void**)&p, sizeof(unsigned long long), cudaHostAllocPortable | cudaHostAllocMapped));
+    *(volatile unsigned long long*)p = ~0ull;  // no round yet
     return 0;
   }
   ~PubLease() {
     if (!p) return;
+    if (!idle) idle = cudaStreamSynchronize(stream) == cudaSuccess;  // a call that ends in an error after its launches
     std::lock_guard<std::mutex> lock(sc->pub_mu);
     (idle ? sc->pub_free : sc->pub_left).push_back(p);
   }
@@ -924,7 +926,7 @@ int launch_wave_step(const Launch& L, const Wave& V, int grid, int block, cudaSt
 }
 
 template <int G>
-int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStream_t stream, int slots_log2,
+int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream, int slots_log2,
              int async, int rounds, float* rpp) {
   const int64_t pool = slots_log2 >= 16 && slots_log2 <= 23 ? (int64_t)1 << slots_log2 : (int64_t)LUMEN_WAVE_POOL;
   int64_t want = L.n < pool ? L.n : pool;
@@ -935,6 +937,8 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
   const size_t npt = sizeof(PhotonTally) / 4;
   const size_t ng = G > 0 ? LUMEN_MAX_GRAD : 0;
   size_t words = (size_t)W * (nph + nex + npt + npre + nq + ng + 3) + 2;
+  if (!async)
+    if (int e = pub.take()) return e;
   uint32_t* buf = nullptr;
   CK(cudaMallocAsync((void**)&buf, words * 4, stream));
   Wave V;
@@ -952,12 +956,8 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
   V.n_in = cnt + 1;
   V.out = list[0];
   V.n_out = cnt;
-  V.pub = nullptr;
   V.round = 0;
-  if (!async && pub) {
-    *(volatile unsigned long long*)pub = ~0ull;
-    V.pub = pub;
-  }
+  V.pub = pub.p;
   const int ext = pk.clip || pk.groups;
   int st = pk.nav64 ? launch_wave_fill<1, 1>(L, V, stream)
                     : (ext ? launch_wave_fill<1, 0>(L, V, stream) : launch_wave_fill<0, 0>(L, V, stream));
@@ -972,7 +972,7 @@ int run_wave(const Launch& L, const Pick& pk, unsigned long long* pub, cudaStrea
   for (;; ++r) {
     if (async && r >= cap) break;
     if (!async && r >= LUMEN_WAVE_AHEAD) {
-      live = wave_seen(pub, r - LUMEN_WAVE_AHEAD, stream);
+      live = wave_seen(pub.p, r - LUMEN_WAVE_AHEAD, stream);
       if (live < 0) {
         CK(cudaStreamSynchronize(stream));
         return set_err(LUMEN_ERR_CUDA, "the wavefront's rounds ended early");

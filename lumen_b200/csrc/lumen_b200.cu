@@ -660,7 +660,7 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
                      cudaStream_t stream, int variant = 0, int bps = 0, int async = 0, int slots_log2 = 0,
                      int rounds = 0, const LumenScene* sc = nullptr) {
   float* rpp = sc ? &sc->wave_rpp : nullptr;
-  PubLease pub(sc);
+  PubLease pub(sc, stream);
   Tally& T = L.T;
   T.E = out ? (out->n_events > 0 ? out->n_events : 1) : (n_events_cot > 0 ? n_events_cot : 1);
   T.S_ = L.R.S.n_sensor > 0 ? L.R.S.n_sensor : 1;
@@ -672,8 +672,6 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
     if (variant == LUMEN_VARIANT_WAVEFRONT) variant = 0;
   }
   if (variant == LUMEN_VARIANT_WAVEFRONT && !async && L.n < LUMEN_WAVE_MIN) variant = 0;  // run_wave's drain alone
-  if (variant == LUMEN_VARIANT_WAVEFRONT && !async)
-    if (int st = pub.take()) return st;
   T.grads = grads;
   // scratch: the photon counter, the abort flag, the steps used and the record count (one small allocation per call)
   const int groups = out && out->n_groups > 0;
@@ -740,11 +738,11 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
         L2.T.counts = (unsigned long long*)(dummy + LUMEN_N_HEALTH);
       }
       st = variant == LUMEN_VARIANT_WAVEFRONT
-               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub.p, stream, slots_log2, async, rounds, rpp)
+               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub, stream, slots_log2, async, rounds, rpp)
                : launch_trace<LUMEN_MAX_GRAD>(L2, pk, variant, bps, stream);
       if (st) return st;
     } else {
-      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub.p, stream, slots_log2, async, rounds, rpp)
+      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub, stream, slots_log2, async, rounds, rpp)
                                               : launch_trace<0>(L, pk, variant, bps, stream);
       if (st) return st;
     }
