@@ -49,8 +49,8 @@ struct LumenScene {
   int lobes;                           // a row draws facets, or a medium has a Mie or WLS channel
   int nav64;                           // LUMEN_PREC_FLOAT64: S's vol_f, node_f, leaf_f, plane_f hold float64 data
   const float* vol_f32;                // the float32 frames (the readout groups' binning reads them in either precision)
-  // the wavefront's rounds per photon a slot carries, from the last synchronous wavefront call (an estimate for the
-  // asynchronous calls' fixed rounds; concurrent calls may overwrite one another's)
+  // the wavefront's rounds per photon a slot carries, from the last synchronous wavefront call of whatever size (an
+  // estimate for the asynchronous calls' fixed rounds; concurrent calls may overwrite one another's)
   mutable float wave_rpp = 0.0f;
   // page-locked words the wavefront's rounds publish their live slots in: one a synchronous call at a time, kept for
   // the scene's later calls (as many as have run at once) and freed with it
@@ -139,6 +139,7 @@ struct Launch {
   unsigned long long* steps_used;
   int budget_chunk;  // steps a thread of the persistent loop counts before it adds them to steps_used (1 .. 256)
   Tally T;
+  unsigned long long* steps;  // the call's steps (an asynchronous call's rounds are estimated from them), or null
   float* truth;  // the photons' analog records (truth rows, LUMEN_F_TRUTH: the ANALOG instantiation), else null
   // the wavefront's live slots a persistent launch resumes before it takes new photons (its drain: thread t the slot
   // wv_list[t], t < *wv_n; wv_W slots in the pool), or wv_W = 0
@@ -493,6 +494,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
     unsigned long long v = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sc[k][w];
     if (v) atomicAdd(L.T.counts + k, v);
+    if (v && k == LUMEN_C_STEPS && L.steps) atomicAdd(L.steps, v);
   }
 }
 
@@ -754,6 +756,7 @@ __global__ void __launch_bounds__(LUMEN_STEP_BLOCK, 512 / LUMEN_STEP_BLOCK) k_wa
     unsigned long long v = 0;
     for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) v += sc[c][w];
     if (v) atomicAdd(L.T.counts + c, v);
+    if (v && c == LUMEN_C_STEPS && L.steps) atomicAdd(L.steps, v);
     if (c == LUMEN_C_STEPS && v && L.step_budget > 0) {  // the call's step budget, counted per block
       unsigned long long used = atomicAdd(L.steps_used, v) + v;
       if (used > (unsigned long long)L.step_budget && atomicExch(L.abort_flag, 1) == 0)
@@ -925,12 +928,25 @@ int launch_wave_step(const Launch& L, const Wave& V, int grid, int block, cudaSt
   return 0;
 }
 
+// The slots of a call of n photons.
+inline int wave_slots(int64_t n, int slots_log2) {
+  const int64_t pool = slots_log2 >= 16 && slots_log2 <= 23 ? (int64_t)1 << slots_log2 : (int64_t)LUMEN_WAVE_POOL;
+  return (int)(((n < pool ? n : pool) + 255) / 256 * 256);
+}
+// The rounds a photon of a slot takes, from the steps of a call whose rounds do not show them (the persistent loop ran it,
+// or its rounds ended at LUMEN_WAVE_MIN live slots): a slot's photons in turn, and the last ones' spread. Rounds until a
+// 64th of the slots are live, over the mean steps a photon: 8.6 at 8 photons a slot (the tank), 2.6 and 1.9 at one (the
+// liquid-argon and the fog box); a round too many costs two launches that find no photon, one too few leaves its photons
+// to the slower drain.
+inline float wave_rounds_of(unsigned long long steps, int64_t n, int64_t W) {
+  const double per_slot = (double)((n + W - 1) / W);
+  return (float)((double)steps / (double)n * (per_slot + 1.5) / per_slot);
+}
+
 template <int G>
 int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream, int slots_log2,
              int async, int rounds, float* rpp) {
-  const int64_t pool = slots_log2 >= 16 && slots_log2 <= 23 ? (int64_t)1 << slots_log2 : (int64_t)LUMEN_WAVE_POOL;
-  int64_t want = L.n < pool ? L.n : pool;
-  int W = (int)((want + 255) / 256 * 256);
+  const int W = wave_slots(L.n, slots_log2);
   const size_t nph = (pk.nav64 ? sizeof(PhotonT<double>) : sizeof(Photon)) / 4, nex = sizeof(WaveExtra) / 4;
   const size_t npre = (pk.nav64 ? sizeof(PreT<double>) : sizeof(Pre)) / 4;
   const size_t nq = (pk.nav64 ? sizeof(WaveQuery<double>) : sizeof(WaveQuery<float>)) / 4;
@@ -965,7 +981,7 @@ int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream
   const long long per_slot = (L.n + W - 1) / W;  // photons a slot carries in turn
   long long cap = -1;                             // rounds of an asynchronous call
   if (async) {
-    const float est = rpp && *rpp > 0.0f ? *rpp : 3.0f;
+    const float est = *rpp > 0.0f ? *rpp : 3.0f;
     cap = rounds > 0 ? rounds : (long long)ceilf(est * (float)per_slot);
   }
   long long r = 0, live = L.n < (int64_t)W ? L.n : W;
@@ -1024,7 +1040,8 @@ int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream
     else st = launch_shape<G, 256, 4, 0>(LD, 0, stream, grid);
     if (st) return st;
   }
-  if (!async && rpp && per_slot > 0) *rpp = (float)r / (float)per_slot;
+  // the rounds a photon of a slot takes, where they ran until a 64th of the slots were live
+  if (!async) *rpp = W / 64 >= LUMEN_WAVE_MIN ? (float)r / (float)per_slot : 0.0f;
   CK(cudaFreeAsync(buf, stream));
   return 0;
 }

@@ -657,9 +657,9 @@ static int check_cells(const Tally& T) {
 }
 
 static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* cot, int n_events_cot, double* grads,
-                     cudaStream_t stream, int variant = 0, int bps = 0, int async = 0, int slots_log2 = 0,
-                     int rounds = 0, const LumenScene* sc = nullptr) {
-  float* rpp = sc ? &sc->wave_rpp : nullptr;
+                     cudaStream_t stream, int variant, int bps, int async, int slots_log2,
+                     int rounds, const LumenScene* sc) {
+  float rpp = sc->wave_rpp;
   PubLease pub(sc, stream);
   Tally& T = L.T;
   T.E = out ? (out->n_events > 0 ? out->n_events : 1) : (n_events_cot > 0 ? n_events_cot : 1);
@@ -671,23 +671,27 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
     L.truth = out->truth;
     if (variant == LUMEN_VARIANT_WAVEFRONT) variant = 0;
   }
+  const int estimate = variant == LUMEN_VARIANT_WAVEFRONT && !async && L.n > 0;  // of an asynchronous call's rounds
   if (variant == LUMEN_VARIANT_WAVEFRONT && !async && L.n < LUMEN_WAVE_MIN) variant = 0;  // run_wave's drain alone
   T.grads = grads;
-  // scratch: the photon counter, the abort flag, the steps used and the record count (one small allocation per call)
+  // scratch: the photon counter, the abort flag, the steps used, the record count and the steps (one small allocation per
+  // call)
+  enum { S_NEXT, S_ABORT, S_USED, S_REC, S_STEPS, S_N };
   const int groups = out && out->n_groups > 0;
   int st0 = 0;
   if (groups && (st0 = check_groups(L.R.S.n_sensor, out))) return st0;
   if ((st0 = check_cells(T))) return st0;
   unsigned long long* scratch = nullptr;
-  CK(cudaMallocAsync((void**)&scratch, 4 * sizeof(unsigned long long), stream));
-  CK(cudaMemsetAsync(scratch, 0, 4 * sizeof(unsigned long long), stream));
-  L.next = scratch;
-  L.abort_flag = (int*)(scratch + 1);
-  L.steps_used = scratch + 2;
+  CK(cudaMallocAsync((void**)&scratch, S_N * sizeof(unsigned long long), stream));
+  CK(cudaMemsetAsync(scratch, 0, S_N * sizeof(unsigned long long), stream));
+  L.next = scratch + S_NEXT;
+  L.abort_flag = (int*)(scratch + S_ABORT);
+  L.steps_used = scratch + S_USED;
+  L.steps = estimate ? scratch + S_STEPS : nullptr;
   if (groups) {
     L.R.rec = (uint32_t*)out->records;
     L.R.rec_cap = out->rec_capacity;
-    L.R.rec_n = scratch + 3;
+    L.R.rec_n = scratch + S_REC;
   }
   // adjoint calls with no tallies of their own accumulate health and counts into the scratch's tail
   double* dummy = nullptr;
@@ -738,11 +742,11 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
         L2.T.counts = (unsigned long long*)(dummy + LUMEN_N_HEALTH);
       }
       st = variant == LUMEN_VARIANT_WAVEFRONT
-               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub, stream, slots_log2, async, rounds, rpp)
+               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub, stream, slots_log2, async, rounds, &rpp)
                : launch_trace<LUMEN_MAX_GRAD>(L2, pk, variant, bps, stream);
       if (st) return st;
     } else {
-      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub, stream, slots_log2, async, rounds, rpp)
+      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub, stream, slots_log2, async, rounds, &rpp)
                                               : launch_trace<0>(L, pk, variant, bps, stream);
       if (st) return st;
     }
@@ -758,14 +762,17 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
     if (dummy) CK(cudaFreeAsync(dummy, stream));
     return 0;
   }
-  int flag = 0;
-  unsigned long long n_rec = 0;
-  CK(cudaMemcpyAsync(&flag, L.abort_flag, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  CK(cudaMemcpyAsync(&n_rec, scratch + 3, sizeof(n_rec), cudaMemcpyDeviceToHost, stream));
+  unsigned long long end[S_N];
+  CK(cudaMemcpyAsync(end, scratch, sizeof(end), cudaMemcpyDeviceToHost, stream));
   CK(cudaFreeAsync(scratch, stream));
   if (dummy) CK(cudaFreeAsync(dummy, stream));
   CK(cudaStreamSynchronize(stream));
   pub.idle = 1;
+  const int flag = *(const int*)(end + S_ABORT);
+  const unsigned long long n_rec = end[S_REC];
+  if (estimate && !flag)
+    sc->wave_rpp = variant == LUMEN_VARIANT_WAVEFRONT && rpp > 0.0f
+                       ? rpp : wave_rounds_of(end[S_STEPS], L.n, wave_slots(L.n, slots_log2));
   if (flag) return set_err(LUMEN_ERR_STEP_BUDGET, "the call's step budget ran out before every photon ended");
   if (groups && n_rec > (unsigned long long)out->rec_capacity)
     return set_err(LUMEN_ERR_RECORDS, "the deposit records outgrew rec_capacity (" + std::to_string(n_rec) +

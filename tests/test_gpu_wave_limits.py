@@ -1,8 +1,11 @@
-"""The wavefront at the limits of what a call holds beside its tallies: its page-locked word over refused calls."""
+"""The wavefront at the limits of what a call holds beside its tallies: its page-locked word over refused calls,
+and the rounds of an asynchronous call after small synchronous ones."""
 
 import ctypes
 
+import numpy as np
 import pytest
+import torch
 
 from lumen_b200 import _abi as A
 from lumen_b200 import detectors, sources
@@ -48,3 +51,21 @@ def test_refused_calls_keep_no_page_locked_memory():
     eng.trace((0, 1), 1 << 14, source=ds, controls=c, tallies=T)
     assert int(T.counts[A.C_PHOTONS]) == 1 << 14
     assert grown < 4096, f"{grown} kB"
+
+
+@pytest.mark.parametrize("n", [4096, 16384])
+def test_rounds_of_an_asynchronous_call_after_a_small_one(n):
+    """An asynchronous call takes its rounds from the scene's last synchronous wavefront call, a small one too (one the
+    persistent loop ran, or whose rounds ended well before a 64th of its slots were live): the liquid-argon box's photons
+    take some 48 steps each."""
+    eng, ds, T = _setup("lar_box", (0.2, 0.3, 0.1), 1 << 16)
+    eng.trace((0, 1), n, source=ds, controls=A.controls(variant=A.VARIANT_WAVEFRONT), tallies=T)
+    steps = float(T.counts[A.C_STEPS]) / n
+    assert steps > 20.0
+    T.zero_()
+    eng.trace((0, 1), 1 << 16, source=ds, tallies=T, controls=A.controls(variant=A.VARIANT_WAVEFRONT, flags=A.F_ASYNC))
+    launches = eng.launches
+    torch.cuda.synchronize()
+    assert int(T.counts[A.C_PHOTONS]) == 1 << 16
+    assert 2 * 1.5 * steps < launches < 2 * 5.0 * steps, (launches, steps)
+    assert np.isfinite(T.health.cpu().numpy()).all()
