@@ -28,7 +28,10 @@ inline int set_err(int code, const std::string& m) {
 #define CK(call)                                                                               \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
-    if (e_ != cudaSuccess) return set_err(LUMEN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                                   \
+      cudaGetLastError(); /* not the next launch's */                                          \
+      return set_err(LUMEN_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
+    }                                                                                          \
   } while (0)
 
 struct LumenScene {
@@ -880,6 +883,7 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 #define LUMEN_WAVE_POOL (1 << 21)
 #define LUMEN_WAVE_AHEAD 2
 #define LUMEN_WAVE_MIN 8192
+#define LUMEN_WAVE_NO_SLOTS (-1)  // run_wave: no memory for the slots, nothing launched (the persistent loop needs none)
 
 // threads a block for n live slots: whole blocks of 256 while they fill the chip several times over, fewer where that
 // leaves SMs without one (148 SMs). Large blocks are the better ones: their warps start together and share the
@@ -956,7 +960,12 @@ int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream
   if (!async)
     if (int e = pub.take()) return e;
   uint32_t* buf = nullptr;
-  CK(cudaMallocAsync((void**)&buf, words * 4, stream));
+  const cudaError_t full = cudaMallocAsync((void**)&buf, words * 4, stream);
+  if (full == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return LUMEN_WAVE_NO_SLOTS;
+  }
+  CK(full);
   Wave V;
   V.W = W;
   V.ph = buf;

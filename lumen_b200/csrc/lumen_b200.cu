@@ -656,6 +656,18 @@ static int check_cells(const Tally& T) {
   return 0;
 }
 
+// the call's launches in its variant; a wavefront whose slots find no memory runs as the persistent loop
+template <int G>
+static int run_wave_or_loop(const Launch& L, const Pick& pk, PubLease& pub, int& variant, int bps, cudaStream_t stream,
+                            int slots_log2, int async, int rounds, float* rpp) {
+  if (variant == LUMEN_VARIANT_WAVEFRONT) {
+    const int st = run_wave<G>(L, pk, pub, stream, slots_log2, async, rounds, rpp);
+    if (st != LUMEN_WAVE_NO_SLOTS) return st;
+    variant = 0;
+  }
+  return launch_trace<G>(L, pk, variant, bps, stream);
+}
+
 static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* cot, int n_events_cot, double* grads,
                      cudaStream_t stream, int variant, int bps, int async, int slots_log2,
                      int rounds, const LumenScene* sc) {
@@ -741,14 +753,9 @@ static int run_trace(Launch& L, Pick pk, const LumenTallies* out, const double* 
         L2.T.health = dummy;
         L2.T.counts = (unsigned long long*)(dummy + LUMEN_N_HEALTH);
       }
-      st = variant == LUMEN_VARIANT_WAVEFRONT
-               ? run_wave<LUMEN_MAX_GRAD>(L2, pk, pub, stream, slots_log2, async, rounds, &rpp)
-               : launch_trace<LUMEN_MAX_GRAD>(L2, pk, variant, bps, stream);
-      if (st) return st;
+      if ((st = run_wave_or_loop<LUMEN_MAX_GRAD>(L2, pk, pub, variant, bps, stream, slots_log2, async, rounds, &rpp))) return st;
     } else {
-      st = variant == LUMEN_VARIANT_WAVEFRONT ? run_wave<0>(L, pk, pub, stream, slots_log2, async, rounds, &rpp)
-                                              : launch_trace<0>(L, pk, variant, bps, stream);
-      if (st) return st;
+      if ((st = run_wave_or_loop<0>(L, pk, pub, variant, bps, stream, slots_log2, async, rounds, &rpp))) return st;
     }
   }
   if (ev_vol) CK(cudaFreeAsync(ev_vol, stream));

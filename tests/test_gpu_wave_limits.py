@@ -1,7 +1,9 @@
-"""The wavefront at the limits of what a call holds beside its tallies: its page-locked word over refused calls,
-and the rounds of an asynchronous call after small synchronous ones."""
+"""The wavefront at the limits of what a call holds beside its tallies: its page-locked word over refused calls, its slots
+over the device memory that is free, and the rounds of an asynchronous call after small synchronous ones."""
 
 import ctypes
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -51,6 +53,49 @@ def test_refused_calls_keep_no_page_locked_memory():
     eng.trace((0, 1), 1 << 14, source=ds, controls=c, tallies=T)
     assert int(T.counts[A.C_PHOTONS]) == 1 << 14
     assert grown < 4096, f"{grown} kB"
+
+
+LOW = """
+import sys, torch
+from lumen_b200 import _abi as A, detectors, sources
+from lumen_b200.engine import DeviceSource, DeviceTallies, Engine
+n = 1 << 20
+det = detectors.coated_panel().with_precision("float64")
+eng, src = Engine(det), sources.Point(position=(4.0, 0.1, 0.1), n_photons=1.0, lam=420.0)
+ds, T, cot = DeviceSource(src, n), DeviceTallies(det.n_sensor), torch.ones(1, det.n_sensor, dtype=torch.float64, device="cuda")
+def run(n, grads=(), **kw):
+    c = A.controls(grad_tabs=[det.params_index[g] for g in grads], **kw)
+    T.zero_()
+    if grads:
+        return eng.adjoint((0, 5), n, cot, source=ds, controls=c).tolist()
+    eng.trace((0, 5), n, source=ds, controls=c, tallies=T)
+    return T.counts.tolist()[:4]
+W = A.VARIANT_WAVEFRONT
+grads = ["media/Water/absorption"]
+for v in (0, W):  # what the kernels themselves hold on the device (their stacks)
+    run(9000, variant=v), run(9000, grads, variant=v)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+hog = torch.empty(torch.cuda.mem_get_info()[0] - (150 << 20), dtype=torch.uint8, device="cuda")
+low = [run(n, variant=W), run(n, grads, variant=W), run(n, variant=W, wave_slots_log2=23)]
+torch.cuda.synchronize()
+del hog
+torch.cuda.empty_cache()
+want = [run(n, variant=0), run(n, grads, variant=0)]
+assert low[0] == want[0] and low[2] == want[0], (low, want)
+assert abs(low[1][0] - want[1][0]) <= 1e-7 * abs(want[1][0]), (low, want)
+print("ok", low)
+"""
+
+
+def test_slots_past_the_free_memory():
+    """A call whose slots (some 400 bytes a photon in flight) do not fit into the memory left still runs, as it does in
+    the persistent loop, and so does the next: the float64 panel with 150 MB free, forward and adjoint."""
+    from lumen_b200 import make
+
+    make.build()
+    r = subprocess.run([sys.executable, "-c", LOW], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout + r.stderr[-3000:]
 
 
 @pytest.mark.parametrize("n", [4096, 16384])
