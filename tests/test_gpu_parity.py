@@ -90,6 +90,7 @@ def _tallies(det, src, n, controls=None, n_bins=0, pools=None):
     ds = DeviceSource(src, n)
     T = DeviceTallies(det.n_sensor, ds.n_events, n_bins, 0.0, 1.0, c.n_grad)
     eng.trace(KEY, n, source=ds, controls=c, tallies=T)
+    T.launches = eng.launches
     O, _ = oracle.trace(det, KEY, n, source=src, samples=n, controls=c, n_events=ds.n_events, n_bins=n_bins,
                         bin_w=1.0, pool_live=None if pools is None else pools[0],
                         pool_ref=None if pools is None else pools[1])
@@ -227,10 +228,11 @@ def test_wavefront_tallies_match(which, tank, facet_lar, built):
         det = facet_lar
         src = sources.Scintillation(position=[(0.3, 0.2, -0.4), (-1.0, 1.0, 0.5)], lam=128.0, tau=(6.0, 1500.0),
                                     fraction=0.25)  # fmt: skip
-        names, n = ["surfaces/CageSurface/R", "media/LAr/rayleigh"], 1 << 12
+        names, n = ["surfaces/CageSurface/R", "media/LAr/rayleigh"], 1 << 14  # past the calls the persistent loop runs
     for grads in ((), names):
         c = A.controls(grad_tabs=[det.params_index[k] for k in grads], variant=A.VARIANT_WAVEFRONT)
         T, O = _tallies(det, src, n, controls=c, n_bins=50)
+        assert T.launches >= 8  # the locate, the fill, at least two rounds of two kernels, the drain, the moments
         np.testing.assert_allclose(T.arrival.cpu().numpy(), O.arrival, rtol=RTOL, atol=1e-15)
         np.testing.assert_allclose(T.arrival2.cpu().numpy(), O.arrival2, rtol=RTOL, atol=1e-15)
         np.testing.assert_allclose(T.hist.cpu().numpy(), O.hist, rtol=RTOL, atol=1e-12)
@@ -553,7 +555,7 @@ def test_float64_tallies_gradients_and_truth(tank, toy, built):
     det = tank.with_precision("float64")
     src = sources.Point(position=(1.0, -0.5, 2.0), n_photons=1.0, lam_range=(300.0, 600.0))
     grads = [det.params_index[k] for k in ("media/Water/absorption", "media/Water/rayleigh")]
-    c = A.controls(grad_tabs=grads, variant=3)  # a wavefront request runs the persistent loop in float64
+    c = A.controls(grad_tabs=grads, variant=A.VARIANT_WAVEFRONT)
     T, O = _tallies(det, src, 1 << 15, controls=c)
     np.testing.assert_allclose(T.arrival.cpu().numpy(), O.arrival, rtol=RTOL, atol=1e-15)
     np.testing.assert_allclose(T.jac.cpu().numpy(), O.jac, rtol=1e-7, atol=1e-12)

@@ -89,7 +89,7 @@ print("ok", low)
 
 
 def test_slots_past_the_free_memory():
-    """A call whose slots (some 400 bytes a photon in flight) do not fit into the memory left still runs, as it does in
+    """A call whose slots (316 or 348 bytes a photon in flight) do not fit into the memory left still runs, as it does in
     the persistent loop, and so does the next: the float64 panel with 150 MB free, forward and adjoint."""
     from lumen_b200 import make
 

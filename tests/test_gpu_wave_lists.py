@@ -34,6 +34,10 @@ def _run(eng, name, n, grads=(), **kw):
     T = DeviceTallies(det.n_sensor, 1, 0, 0.0, 1.0, len(grads))
     c = A.controls(grad_tabs=[det.params_index[g] for g in grads], **kw)
     eng.trace((0, 5), n, source=DeviceSource(src, n), controls=c, tallies=T)
+    if kw.get("variant") == A.VARIANT_WAVEFRONT and n >= 8192:  # the fill, two rounds or more, the drain, the moments
+        assert eng.launches >= 7
+    else:
+        assert eng.launches <= 3
     return T
 
 
