@@ -39,9 +39,9 @@ L2_FLUSH_BYTES = 256 << 20
 
 # DRAM bytes per photon-step of the tank workload, from ncu's dram__bytes_read.sum + dram__bytes_write.sum: the
 # persistent loop k_trace<0,256,4,2,0,0> on one launch of 2^20 photons (2.76 steps each; local memory almost all of
-# it), and the wavefront's k_wave_query<0,2> + k_wave_step<0> summed over every round of seven calls of 2^20 photons
-# (2.76 steps each; 2.613 GB read + 2.090 GB written per call: the slots' state and the kernels' local memory)
-TRAFFIC_PER_STEP = {0: (0.253087e9 + 1.570654e9) / (1048576 * 2.760), 3: (2.613e9 + 2.090e9) / (1048576 * 2.760)}
+# it), and the wavefront's fill, queries, steps and drain summed over nine calls of 2^20 photons (2.005 GB read + 0.841 GB
+# written per call: the slots' state and the kernels' local memory)
+TRAFFIC_PER_STEP = {0: (0.158275e9 + 1.431434e9) / (1048576 * 2.760), 3: (2.0053e9 + 0.8410e9) / (1048576 * 2.760)}
 
 
 def workload_point(seed=12345):

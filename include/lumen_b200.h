@@ -284,9 +284,11 @@ enum { LUMEN_VARIANT_WAVEFRONT = 3, LUMEN_N_VARIANT = 4 };
 /* launch variants: the persistent photon loop at 0 = 256 threads x 4 blocks / SM (64 registers), 1 = 128 x 8 (64),
    2 = 256 x 3 (85 registers); 3 = the wavefront: rounds of two kernels (the query; the rest of the step and the
    refill) over a pool of slots in HBM, then the persistent loop resuming the slots still live (its drain: one thread
-   a slot, then the photons left). A synchronous call reads a live-slot count back every four rounds and drains once
-   fewer than a 64th of the slots are live; a LUMEN_F_ASYNC call runs a fixed number of rounds (wave_rounds) and
-   drains, reading nothing back. Every variant gives the same photons the same paths. */
+   a slot, then the photons left). A synchronous call runs rounds until fewer than a 64th of the slots, or than 8192,
+   are live (each round publishes its live slots to page-locked host memory, which the call reads two rounds behind);
+   one of fewer than 8192 photons, or whose slots find no device memory, runs as variant 0. A LUMEN_F_ASYNC call runs a
+   fixed number of rounds (wave_rounds) and drains, reading nothing back, whatever its photons. Every variant gives the
+   same photons the same paths. */
 typedef struct LumenControls {
   float max_distance;      /* m: a query's reach (<= 0: the scene's reach) */
   float roulette;          /* epsilon > 0 (src/lumen/rules/choices.py:112) */
@@ -301,10 +303,9 @@ typedef struct LumenControls {
                               autotuner: each slot carries n / 2^k photons in turn */
   int32_t wave_rounds;     /* the wavefront's rounds in a LUMEN_F_ASYNC call, which reads no round back: after them
                               the persistent loop finishes the live slots and the photons left (<= 0: the scene's
-                              rounds per photon a slot carries, measured by its last synchronous wavefront call, else
-                              3, times the photons a slot carries). A synchronous call reads the live slots back every
-                              fourth round and hands the tail (fewer than a 64th of the slots live) to the
-                              persistent loop; it ignores this field. */
+                              rounds per photon a slot carries, from its last synchronous call of this variant: counted,
+                              or where the call had too few slots for that estimated from its steps a photon; 3 before
+                              the first; times the photons a slot carries). A synchronous call ignores it. */
 } LumenControls;
 
 /* --------------------------------------------------------------------------------------------- the tallies */
@@ -380,7 +381,8 @@ typedef struct LumenTallies {
 } LumenTallies;
 
 /* ------------------------------------------------------------------------------------------- entry points */
-/* Version of this ABI (LUMEN_B200_ABI_VERSION). */
+/* Version of this ABI (LUMEN_B200_ABI_VERSION): what the structs' layouts and the calls below agree on. An entry point
+   added beside them leaves it; a caller that needs one looks its symbol up. */
 int32_t lumen_b200_abi_version(void);
 /* The last error message of this thread (static storage; "" after success). */
 const char* lumen_b200_last_error(void);

@@ -114,9 +114,10 @@ def simulate(det, source, params=None, *, samples=None, seed=0, reference=None, 
     values the draws are made at (default: ``params``). ``controls``: ``dict(roulette=0.01, max_distance=None,
     max_vertices=2**22, variant=None, jump=True)``; ``jump`` the diffusion jump (on, as lumen.simulate's default: where a
     medium and volume allow it; the same estimator in law as the plain walk); ``variant`` picks the launch
-    (``LumenControls.variant``; default: the wavefront, measured the faster on the tank and LAr workloads, forward and
-    with tangents; scenes it does not serve run the persistent loop). ``chunk``: photons per launch (default: all in one launch). ``gradients``: parameter names
-    whose derivatives of the arrivals are returned (forward tangents of the reweighting estimator along each path).
+    (``LumenControls.variant``; default: the wavefront, measured the faster on every timed workload; calls below 8192
+    photons and truth rows run the persistent loop). ``chunk``: photons per launch (default: all in one launch).
+    ``gradients``: parameter names whose derivatives of the arrivals are returned (forward tangents of the reweighting
+    estimator along each path).
     ``time_bins``: (bins, t0, width) ns of the per-sensor arrival-time histograms (``Light.diagnostics``).
     ``groups``: the readout groups' histograms to fill ({name: lumen_b200.readout.Grid or Group}: a Grid's sensors
     are the detector's group of that name, else every sensor) into ``Light.groups`` (src/lumen/readout/grid.py

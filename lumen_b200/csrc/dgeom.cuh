@@ -48,10 +48,11 @@ struct DScene {
   const float* __restrict__ node_f;
   const int32_t* __restrict__ node_i;
   const int32_t* __restrict__ items;
-  // the float32 ray traversal's node records, 16 words a node: an inner node's left and right child boxes (lo, hi:
-  // words 0-5 and 6-11) and codes (12, 13), every node's own code (14); a code is an inner node's index or -2 - p for
-  // a leaf whose items are witem[p], witem[p + 1], ... up to a -1. A volume's records lie in its node range, the root
-  // first; their tree is scene_create's own over the BVH's leaves (ray_records)
+  // the float32 ray traversal's records, 16 words each: an inner node's left and right child boxes (lo, hi: words 0-5
+  // and 6-11) and codes (12, 13), its own code (14); a code is an inner node's record or -2 - p for a leaf whose items
+  // are witem[p], witem[p + 1], ... up to a -1. scene_create builds a tree of its own over the leaves of each volume's
+  // BVH (ray_records): its root is the record at the volume's first node (a leaf's code there where it is the only one),
+  // its other inner nodes lie after the scene's n_node records; the other nodes' records are not read
   const float4* __restrict__ node_w;
   const int32_t* __restrict__ witem;
   const int32_t* __restrict__ kind_i;

@@ -23,9 +23,8 @@
 
 // loops whose count is the call's or the data's stay rolled: the compiler's copies by four were most of a kernel's code,
 // and the kernels wait on instruction fetch (the step kernel with tangents 10 stalls an issue on it). With the settle's
-// solids read in the scene's own instantiation (dnav.cuh d_ray_holds), same box, ms: the tank's 2^24 photons 43.1 -> 40.0,
-// the ground-wall tank with four tangents 12.6 -> 11.3, the track events 14.1 -> 13.3, the liquid-argon box 25.0 -> 23.9,
-// the readout tank 8.8 -> 8.1, the solids box 9.6 -> 8.6, the float64 panel 4.2 -> 4.0
+// solids read in the scene's own instantiation (dnav.cuh d_ray_holds), ms: the tank's 2^24 photons 43.1 -> 40.0, the
+// ground-wall tank with four tangents 12.6 -> 11.3; the other scenes 4 to 10 % faster
 #define L_ROLL _Pragma("unroll 1")
 // the elementary functions: inlined, or one copy a kernel where the part says so (k_part.cu)
 #ifndef L_MATH

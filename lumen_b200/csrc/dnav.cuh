@@ -1231,10 +1231,9 @@ L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {
 // 16-byte loads a level), apart from the visits: the leaves a ray meets are set aside, up to D_CAND of them, and visited
 // once the walk has ended or the list is full, those past an event found since left out. A warp's lanes meet their leaves
 // after different numbers of nodes; visited as they were met, the warp waited for its slowest lane's next leaf before
-// each visit. The votes hold the lanes that entered together to one node, and to one visit, at a time: without
-// them the compiler's branches let the lanes run apart (7 of 32 lanes an instruction on the tank, 16 in the loop that
-// visited as it walked, 20 here; its 2^24 photons 55.6, 40.1 and 39.0 ms). Lists of 4 measured the same, visits at the
-// first leaf (with votes) 42.0 ms.
+// each visit. The votes hold the lanes that entered together to one node, and to one visit, at a time: without them the
+// compiler's branches let the lanes run apart (7 of 32 lanes an instruction on the tank, 20 with them; 55.6 and 39.0 ms
+// for its 2^24 photons; 40.1 in a loop that visits as it walks).
 #define D_CAND 6
 template <int TORUS>
 L_DEV Best d_enter(const DScene& S, const Ctx& c, int has_own, int vi) {

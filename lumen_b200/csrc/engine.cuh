@@ -507,23 +507,19 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_trace(Launch L) {
 // the step, the deposit, the photon's end and the slot's refill from the source. Each kernel is a part of the
 // megakernel's code with its own registers; the state crosses HBM between them, word-major (word k of slot i at
 // buf[k * W + i]) so that the loads and stores of neighbouring slots are contiguous. A round moves what it must: the
-// query stores the photon only where its start changed it (131 words a step instead of 218), and of its result what the
-// step reads; the step's sensor sums are read where it deposits or ends. With the hit's gradient kept from the settle
-// (dnav.cuh), same box, ms: tank 2^24 photons 39.1 -> 35.1, 1,000,003 3.22 -> 2.86, ground wall with four tangents 10.3
-// -> 9.7, track events 12.8 -> 11.4, liquid-argon box 23.5 -> 21.8, float64 panel 3.93 -> 3.20, solids box 8.6 -> 8.2.
+// query stores the photon only where its start changed it, and of its result what the step reads; the step reads the
+// sensor sums where it deposits or ends (131 words a step; with all 218 and the hit's gradient taken twice the tank's 2^24
+// photons took 39.1 instead of 35.1 ms).
 //
 // The kernels run over lists of live slots, not over the pool: once the source is spent a photon's end leaves its lane
-// idle for every later round, and with one photon a slot that is from the second round on (measured before the lists:
-// half of the step kernel's lanes in the liquid-argon box and the fog box, a third in the tank). The step kernel
-// appends the slots that go on to the next round's list, and the query kernel orders each block's slots by the event it
-// found, scatterings ahead of crossings, so that all but one warp of a block of the step kernel run one side of that
-// branch. Both keep a block's slots together and in order: neighbours in a list are neighbours in the pool, and a
-// warp's words stay in few sectors (a split of the whole list, which scatters it round by round, took 129 ms instead of
-// 45 for the tank's 2^24 photons).
+// idle for every later round, and with one photon a slot that is from the second round on. The step kernel appends the
+// slots that go on to the next round's list, and the query kernel orders each block's slots by the event it found,
+// scatterings ahead of crossings, so that all but one warp of a block of the step kernel run one side of that branch. Both
+// keep a block's slots together and in order: neighbours in a list are neighbours in the pool, and a warp's words stay in
+// few sectors (a split of the whole list scatters them round by round: the tank's 2^24 photons 129 instead of 45 ms).
 //
 // EXT: the locate of scenes with protrusion clips or frame groups; NAV64: the float64 navigator's records. Every scene
-// runs here: the solids box (clips) 100,003 photons 20.2 ms in the persistent loop, 9.4 in the wavefront; the coated
-// panel (float64) 2^20 photons 7.0 and 4.2 ms.
+// runs here (the solids box, with clips, 100,003 photons: 20.2 ms in the persistent loop, 9.4 in the wavefront).
 template <int EXT, class NF>
 __device__ __forceinline__ void wave_new(const Launch& L, int64_t g, PhotonT<NF>& ph, WaveExtra& ex) {
   Row r;
@@ -865,33 +861,33 @@ int launch_shape(const Launch& L, int bps, cudaStream_t stream, int blocks) {
 // The wavefront's rounds (LUMEN_VARIANT_WAVEFRONT): a fill, then query and step kernels, then the drain: the
 // persistent loop resumes every slot still live (one thread a slot) and takes the photons left. Each round's query
 // writes its live slots to page-locked host memory as it starts (`pub`), and a synchronous call launches round r once
-// it has seen round r - LUMEN_WAVE_AHEAD's: no round waits for the host, the grids follow the live slots down (they
-// only ever fall), and the drain starts once fewer than a 64th of the slots, or than LUMEN_WAVE_MIN, are live: a round is
-// two launches that wait for their slowest photon, and below some 8192 photons, 2 warps a scheduler, that wait is all
-// there is (a call of fewer photons runs the persistent loop from the start). Drain below a 64th, 2048, 4096, 8192,
-// 16384, same box, ms: liquid-argon box 21.5, 21.2, 20.7, 20.2, 20.7; solids box 8.1, 8.2, 7.8, 7.6, 7.2; fog box 9.4,
-// 8.7, 8.2, 8.1, 8.8; the others within 1 %. The whole call, persistent loop against wavefront, at 1024, 4096-8192 and
-// 16384 photons: tank 0.57 / 1.12, -, 0.72 / 0.74; liquid-argon box -, 9.8 / 13.3, 26 / 15; solids box 2.9 / 4.5,
-// 4.6 / 5.7, -; fog box 4.0 / 6.5, -, 8.9 / 8.2; toy tank -, 0.42 / 0.46, 0.47 / 0.47 (32768). An asynchronous call
-// (LUMEN_F_ASYNC) runs `rounds` rounds over the whole pool without a readback (<= 0: *rpp rounds per photon a slot
-// carries, the scene's estimate from its last synchronous call) and drains. Against rounds over the whole pool with a
-// readback every fourth (2^24 photons of the tank 45.5 -> 43.6 ms, 1,000,003 5.08 -> 3.83, the ground-wall tank with
-// four tangents 19.7 -> 13.1, the track events 19.9 -> 16.1, the liquid-argon box's 131,072 48 -> 41, the readout tank's
-// 300,007 11.2 -> 9.2); draining at a 256th of the slots, at 2048 or at 64 of them, or looking one or three rounds ahead
-// measured the same within 3 %. The pool holds up to LUMEN_WAVE_POOL slots
-// (about 360 bytes each with gradients), allocated on the call's stream.
+// it has seen round r - LUMEN_WAVE_AHEAD's: no round waits for the host, and the grids follow the live slots down (they
+// only ever fall). The drain starts once fewer than a 64th of the slots, or than LUMEN_WAVE_MIN, are live: a round is two
+// launches that wait for their slowest photon, and below some 8192 photons, 2 warps a scheduler, that wait is all there
+// is. Drain below 2048, 8192, 16384, ms: liquid-argon box 21.2, 20.2, 20.7; fog box 8.7, 8.1, 8.8; solids box 8.2, 7.6,
+// 7.2; the others within 1 %. A call of fewer photons runs the persistent loop from the start (persistent loop against
+// wavefront, ms: liquid-argon box 9.8 and 13.3 at 4096 photons, 26 and 15 at 16,384; fog box 4.0 and 6.5 at 1024, 8.9 and
+// 8.2 at 16,384; tank 0.57 and 1.12 at 1024, 0.72 and 0.74 at 16,384).
+// An asynchronous call (LUMEN_F_ASYNC) runs `rounds` rounds over the whole pool without a readback (<= 0: *rpp rounds per
+// photon a slot carries, the scene's estimate from its last synchronous call) and drains. The pool holds up to
+// LUMEN_WAVE_POOL slots, allocated on the call's stream: 292 bytes a slot, 324 with gradients (316 and 348 in float64).
 #define LUMEN_WAVE_POOL (1 << 21)
 #define LUMEN_WAVE_AHEAD 2
 #define LUMEN_WAVE_MIN 8192
 #define LUMEN_WAVE_NO_SLOTS (-1)  // run_wave: no memory for the slots, nothing launched (the persistent loop needs none)
 
-// threads a block for n live slots: whole blocks of 256 while they fill the chip several times over, fewer where that
-// leaves SMs without one (148 SMs). Large blocks are the better ones: their warps start together and share the
-// instruction fetch that the step waits on (step blocks of 256, 128, 64, 32, same box, ms: tank 2^24 photons 35.2, 40.5,
-// 44.0, 46.6; ground wall with four tangents 9.8, 10.9, 11.6, 11.9; readout tank 7.6, 8.9, 9.3, 9.5). Where the step's
-// code is longest, in scenes that draw facets or have a Mie or WLS channel, it runs in blocks of 512, one an SM (ground
-// wall 9.85 -> 8.98, readout tank 7.63 -> 6.79; the polished tank's 1,000,003 photons lose 1 % in them)
-inline int wave_block(unsigned n) { return n >= 148u * 256u * 4u ? LUMEN_QUERY_BLOCK : (n >= 148u * 128u * 2u ? 128 : (n >= 148u * 64u ? 64 : 32)); }
+// B200's SMs: the launch shapes below were measured on them (any grid runs the same photons)
+#define LUMEN_SMS 148
+// threads a block for n live slots: blocks of 256 while they fill the chip several times over, fewer where that leaves SMs
+// without one. On full chips large blocks are the step's better ones: their warps start together and share the instruction
+// fetch that it waits on (step blocks of 256, 128, 64, ms: tank 2^24 photons 35.2, 40.5, 44.0; ground wall with four
+// tangents 9.8, 10.9, 11.6). Below 4 blocks an SM it hardly matters: query and step in blocks of 64, 128 or 256 measured
+// within 4 % of this rule, to either side, on the timed scenes at 16,384 to 131,072 photons. Where the step's code is
+// longest, in scenes that draw facets or have a Mie or WLS channel, it runs in blocks of 512, one an SM, on full chips
+// (ground wall 9.85 -> 8.98, readout tank 7.63 -> 6.79; below 4 blocks an SM 1 to 7 % slower, the readout tank 4 % faster).
+inline int wave_block(unsigned n) {
+  return n >= LUMEN_SMS * 256u * 4u ? LUMEN_QUERY_BLOCK : (n >= LUMEN_SMS * 128u * 2u ? 128 : (n >= LUMEN_SMS * 64u ? 64 : 32));
+}
 
 // waits for a published round >= `want`; returns its live slots, or -1 where the stream failed
 inline long long wave_seen(volatile unsigned long long* pub, long long want, cudaStream_t stream) {
@@ -1038,7 +1034,7 @@ int run_wave(const Launch& L, const Pick& pk, PubLease& pub, cudaStream_t stream
     LD.wv_W = W;
     // one thread a slot, over as many SMs as there are warps of them
     const long long most = async ? W : live;
-    const int grid = (int)std::max((most + 255) / 256, std::min((most + 31) / 32, 148LL));
+    const int grid = (int)std::max((most + 255) / 256, std::min((most + 31) / 32, (long long)LUMEN_SMS));
     if (pk.nav64)
       st = pk.single ? launch_shape<G, 256, 4, 2, 0, 1>(LD, 0, stream, grid)
                      : (pk.groups ? launch_shape<G, 256, 4, 3, 0, 1>(LD, 0, stream, grid)

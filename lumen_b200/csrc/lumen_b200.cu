@@ -131,8 +131,10 @@ static std::vector<uint32_t> truth_tables(const LumenSceneDesc* d) {
 // The ray traversal's own tree over the leaves of each volume's BVH, in the node records of DScene::node_w (root at
 // the volume's first node, the other inner nodes after the scene's): built by the surface area heuristic, which takes
 // the expected box tests of a random ray instead of the equal halves a caller's tree may have. The queries find the
-// same event over any tree (every leaf box a ray meets before the best event is visited); the boxes are the leaves'
-// own. No deeper than the traversal's stack: a split that could not finish within it is the median's.
+// same event over any tree where the events differ in t (every leaf box a ray meets before the best event is visited) and
+// where volumes tie (the rank decides); of two mesh triangles of different chunks met at the same t, and of a clip's exit
+// at the t of an entry of no higher rank, the first visited wins, and the order of the visits is this tree's. The boxes
+// are the leaves' own. No deeper than the traversal's stack: a split that could not finish within it is the median's.
 struct RayTree {
   struct Box { float v[6]; };
   std::vector<Box> box;
@@ -1189,7 +1191,7 @@ int32_t lumen_b200_finish(LumenTallies* t, int32_t n_sensor, int32_t n_grad, con
   const size_t cells = (size_t)T.E * T.S_, most = cells * (size_t)std::max(1, std::max(T.nb, T.P));
   const size_t want = (most + 255) / 256;
   CK(cudaMemsetAsync(nonfinite, 0, sizeof(double), (cudaStream_t)stream));
-  k_finish<<<(unsigned)std::min<size_t>(want, 148 * 8), 256, 0, (cudaStream_t)stream>>>(T, ev_first, samples, nonfinite);
+  k_finish<<<(unsigned)std::min<size_t>(want, LUMEN_SMS * 8), 256, 0, (cudaStream_t)stream>>>(T, ev_first, samples, nonfinite);
   CK(cudaGetLastError());
   ++lumen_launches();
   return 0;
