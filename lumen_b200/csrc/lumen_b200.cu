@@ -138,8 +138,11 @@ static std::vector<uint32_t> truth_tables(const LumenSceneDesc* d) {
 struct RayTree {
   struct Box { float v[6]; };
   std::vector<Box> box;
-  std::vector<int> code, weight, id;
+  std::vector<int> code, weight;
   std::vector<float>* rec;
+  std::vector<int> ord[3], tmp;  // the leaves in each axis' order of their centres; a node's are [a, b) of all three
+  std::vector<char> left;
+  std::vector<double> right;
 
   static Box none() {
     const float i = std::numeric_limits<float>::infinity();
@@ -160,37 +163,46 @@ struct RayTree {
     while (((long long)1 << (l - 1)) < m) ++l;
     return l;
   }
-  double centre(int i, int ax) const {
-    const double c = 0.5 * ((double)box[i].v[ax] + box[i].v[3 + ax]);
-    return c == c ? c : 0.0;  // (-inf, inf)
-  }
-  void order(int a, int b, int ax) {
-    std::sort(id.begin() + a, id.begin() + b, [&](int p, int q) {
-      const double cp = centre(p, ax), cq = centre(q, ax);
-      return cp != cq ? cp < cq : p < q;
-    });
+
+  // the tree over all leaves (at least two), its root's record at `at`; the orders are made once, and each node hands its
+  // children their parts of all three
+  void build(int at) {
+    const int n = (int)box.size();
+    tmp.resize(n);
+    left.resize(n);
+    right.resize(n);
+    std::vector<double> c(n);
+    for (int ax = 0; ax < 3; ++ax) {
+      ord[ax].resize(n);
+      for (int i = 0; i < n; ++i) {
+        ord[ax][i] = i;
+        c[i] = 0.5 * ((double)box[i].v[ax] + box[i].v[3 + ax]);
+        if (c[i] != c[i]) c[i] = 0.0;  // (-inf, inf)
+      }
+      std::sort(ord[ax].begin(), ord[ax].end(), [&](int p, int q) { return c[p] != c[q] ? c[p] < c[q] : p < q; });
+    }
+    node(0, n, at, 1);
   }
 
-  // writes the record of the inner node over id[a, b) (at least two leaves) at record `at` and returns its box
-  Box build(int a, int b, int at, int level) {
+  // writes the record of the inner node over the leaves [a, b) (at least two) at record `at` and returns its box
+  Box node(int a, int b, int at, int level) {
     const int n = b - a;
     int split = a + n / 2, best_ax = -1;
     double best = std::numeric_limits<double>::infinity();
-    std::vector<double> right(n);
     for (int ax = 0; ax < 3; ++ax) {
-      order(a, b, ax);
+      const int* id = ord[ax].data() + a;
       Box r = none();
       double wr = 0.0;
       for (int i = n - 1; i > 0; --i) {
-        grow(r, box[id[a + i]]);
-        wr += weight[id[a + i]];
+        grow(r, box[id[i]]);
+        wr += weight[id[i]];
         right[i] = area(r) * wr;
       }
       Box l = none();
       double wl = 0.0;
       for (int i = 1; i < n; ++i) {
-        grow(l, box[id[a + i - 1]]);
-        wl += weight[id[a + i - 1]];
+        grow(l, box[id[i - 1]]);
+        wl += weight[id[i - 1]];
         const double cost = area(l) * wl + right[i];
         if (cost < best && level + levels(std::max(i, n - i)) <= LUMEN_MAX_BVH_DEPTH) {
           best = cost;
@@ -199,8 +211,18 @@ struct RayTree {
         }
       }
     }
-    if (best_ax < 0) best_ax = 2;  // the last axis' order is there: the median
-    if (best_ax != 2) order(a, b, best_ax);
+    if (best_ax < 0) best_ax = 2;  // the median of the last axis' order
+    for (int i = a; i < b; ++i) left[ord[best_ax][i]] = i < split;
+    for (int ax = 0; ax < 3; ++ax) {
+      if (ax == best_ax) continue;
+      int* id = ord[ax].data();
+      int p = a, q = 0;
+      for (int i = a; i < b; ++i) {
+        if (left[id[i]]) id[p++] = id[i];
+        else tmp[q++] = id[i];
+      }
+      std::copy(tmp.begin(), tmp.begin() + q, id + p);
+    }
     Box all = none();
     float r[16];
     memset(r, 0, sizeof(r));
@@ -209,12 +231,12 @@ struct RayTree {
       Box bx;
       int c;
       if (q - p == 1) {
-        bx = box[id[p]];
-        c = code[id[p]];
+        bx = box[ord[0][p]];
+        c = code[ord[0][p]];
       } else {
         c = (int)(rec->size() / 16);
         rec->resize(rec->size() + 16);
-        bx = build(p, q, c, level + 1);
+        bx = node(p, q, c, level + 1);
       }
       memcpy(r + 6 * side, bx.v, sizeof(bx.v));
       memcpy(r + 12 + side, &c, 4);
@@ -250,15 +272,14 @@ static void ray_records(const LumenSceneDesc* d, std::vector<float>& rec, std::v
           std::fill(b.v, b.v + 6, 3e38f);
           break;
         }
-      t.id.push_back((int)t.box.size());
       t.box.push_back(b);
       t.weight.push_back(ni[1]);
       t.code.push_back(-2 - (int)witem.size());
       for (int k = 0; k < ni[1]; ++k) witem.push_back(d->items[ni[2] + k]);
       witem.push_back(-1);
     }
-    if (t.id.size() == 1) memcpy(rec.data() + (size_t)n0 * 16 + 14, &t.code[0], 4);
-    else t.build(0, (int)t.id.size(), n0, 1);
+    if (t.box.size() == 1) memcpy(rec.data() + (size_t)n0 * 16 + 14, &t.code[0], 4);
+    else t.build(n0);
   }
 }
 
